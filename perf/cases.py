@@ -219,7 +219,10 @@ def tolerance(case):
     if path == "layer":
         return {"rel": 1.5e-2, "max": 0.07}  # four matmuls in a row, each result rounded to bfloat16; measured against 64 bits: 4.1e-3, 0.018
     if case.get("out") == "float32":
-        return {"rel": 2e-6, "max": 2e-5}    # fp32 sums of exact products; measured 2.5e-7, 1.6e-6 (and four times more K than there)
+        # fp32 sums of exact products. Tensor cores cut what an addition shifts out instead of rounding it, so the error grows
+        # with K: measured against 64 bits 3.4e-6 at K = 8192, 1.7e-5 at 28672 for one chain of additions (bfloat8_b, 512 rows).
+        rel = 1e-6 + 2.5e-9 * case["k"]
+        return {"rel": rel, "max": 10 * rel}
     return {"rel": 6.5e-3, "max": 0.016}     # one rounding to bfloat16; measured 1.7e-3, 3.9e-3
 
 
