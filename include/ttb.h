@@ -165,15 +165,15 @@ int32_t ttb_unpack_bfp(const void *src_dev, int32_t fmt, void *dst_dev, int32_t 
  *         [1,1,32,N] bias tile row, tt_eager/tt_dnn/op_library/bmm/bmm_op.cpp:859-863).
  *   out:  TTB_BFLOAT16 or TTB_FLOAT32, tiled (or row-major with TTB_MM_OUT_ROW_MAJOR).
  * Block-float weights are expanded to bf16 in shared memory (exact) and multiplied on the tcgen05
- * tensor cores; shapes outside the tensor-core kernels' tiling use a CUDA-core kernel with the same
- * arithmetic. Stands in for tt::operations::primary::matmul and the multi-core-reuse program
+ * tensor cores, bf16 weights go there as they are; shapes outside the tensor-core kernels' tiling use a CUDA-core kernel
+ * with the same arithmetic. Stands in for tt::operations::primary::matmul and the multi-core-reuse program
  * factories (bmm_op.hpp:284-346, bmm_op.cpp:828-1303, and the multi_core_reuse program factories
  * beside them). `workspace` is device scratch of at least ttb_matmul_workspace_bytes() bytes (may be NULL when
  * that is 0); it is only touched between launch and completion of this call on `stream`. Its head holds
  * per-output-tile arrival counters that must be zero when the kernel starts: ttb_matmul clears them with a
  * memset on `stream` unless TTB_MM_WORKSPACE_ZEROED is given. */
 int64_t ttb_matmul_workspace_bytes(int32_t w_dtype, int64_t batch, int64_t M, int64_t K, int64_t N, int32_t flags);
-/* Which kernels ttb_matmul uses for a shape (no GPU needed): out[0] = launches (0: the shape-generic CUDA-core kernel;
+/* Which block-float kernels ttb_matmul uses for a shape (no GPU needed): out[0] = launches (0: none of them, always so for bf16 weights;
  * else tensor-core launches over consecutive row ranges), then per launch its row count and 1 for the prefill kernel, 0
  * for a decode kernel - for as many launches as `out` has room for (out_len >= 5). Decode kernels take up to 256 rows and
  * any N that is a multiple of 32 (blocks of two tile rows when the row count is a multiple of 64 and N a multiple of 128,

@@ -1,6 +1,6 @@
 // C-ABI entry points for matmul / linear and the all-gather layout helper: argument validation and
-// kernel selection. Tensor-core kernels take the shapes their tiling covers; everything else goes to the
-// shape-generic CUDA-core kernel, which computes the same function.
+// kernel selection. Tensor-core kernels take the shapes their tiling covers (block-float weights) or any shape
+// (bfloat16 weights); everything else goes to the shape-generic CUDA-core kernel, which computes the same function.
 #include "common.cuh"
 
 namespace ttb {
@@ -8,6 +8,8 @@ int32_t launch_matmul_generic(const void *a, const void *w, int w_dtype, const v
                               int64_t rows, int64_t K, int64_t N, int act, int flags, cudaStream_t stream);
 int32_t launch_bmm_generic(const void *a, const void *w, int w_dtype, void *out, int out_dtype, int64_t batch, int64_t M, int64_t K,
                            int64_t N, cudaStream_t stream);
+int32_t launch_matmul_bf16(const void *a, const void *w, const void *bias, void *out, int out_dtype, int64_t batch, int64_t rows, int64_t K,
+                           int64_t N, int act, int flags, int *status, cudaStream_t stream);
 bool decode_supported(int w_dtype, int64_t rows, int64_t K, int64_t N);
 int64_t decode_workspace_bytes(int64_t rows, int64_t K, int64_t N, bool smem_operand);
 int32_t launch_matmul_decode(const void *a, const void *w, int w_dtype, const void *bias, void *out, int out_dtype,
@@ -52,6 +54,11 @@ int32_t validate(const void *a, int a_dtype, const void *w, int w_dtype, void *o
         return fail(TTB_E_INVALID, "ttb_matmul: tensors must be 16-byte aligned");
     return TTB_OK;
 }
+
+// bfloat16 weights: the tensor-core kernel, except for fp32 results of fewer than 128 products, where its additions (which
+// cut off low bits) come out further from 64 bits than a chain of fused multiply-adds (2-norm at K = 64: 6.5e-8 against
+// 5.1e-8; at 128: 7.1e-8 against 7.3e-8, and the longer the further ahead).
+bool bf16_on_tensor_cores(int out_dtype, int64_t K) { return out_dtype == TTB_BFLOAT16 || K >= 128; }
 
 // Row ranges of one matmul and the tensor-core kernel that takes each: the decode kernels serve up to 256 rows, the prefill
 // kernel multiples of 128 from 512 up (column counts that are multiples of 128). Row counts in between run as two decode
@@ -113,7 +120,8 @@ int64_t ttb_matmul_workspace_bytes(int32_t w_dtype, int64_t batch, int64_t M, in
     return bytes;
 }
 
-/* Which kernels ttb_matmul would use: out[0] = launches (0: the shape-generic CUDA-core kernel), then per launch its rows
+/* Which block-float kernels ttb_matmul would use: out[0] = launches (0: none of them - the shape-generic CUDA-core kernel, or for
+ * bfloat16 weights usually the kernel of matmul_bf16.cu), then per launch its rows
  * and 1 for the prefill kernel, 0 for a decode kernel - for as many launches as `out` has room for (at least two). */
 int32_t ttb_matmul_plan(int32_t w_dtype, int64_t batch, int64_t M, int64_t K, int64_t N, int32_t flags, int64_t *out, int32_t out_len) {
     if (!out || out_len < 5) return fail(TTB_E_INVALID, "ttb_matmul_plan: needs room for 5 values");
@@ -133,6 +141,11 @@ int32_t ttb_matmul(const void *a, int32_t a_dtype, const void *w, int32_t w_dtyp
     if (int32_t rc = validate(a, a_dtype, w, w_dtype, out, out_dtype, batch, M, K, N, act)) return rc;
     const int64_t rows = batch * M;  // tiled [batch, M, K] with M % 32 == 0 is the same buffer as tiled [batch*M, K]
     auto s = (cudaStream_t)stream;
+    if (w_dtype == TTB_BFLOAT16 && !(flags & TTB_MM_FORCE_GENERIC) && bf16_on_tensor_cores(out_dtype, K) && rows / 32 <= 65535) {
+        int *status = nullptr;
+        if (int32_t rc = status_word_address(&status)) return rc;
+        return launch_matmul_bf16(a, w, bias, out, out_dtype, 1, rows, K, N, act, flags, status, s);
+    }
     RowChunk chunks[kMaxRowChunks];
     const int n = (flags & TTB_MM_FORCE_GENERIC) ? 0 : plan_rows(w_dtype, rows, K, N, chunks);
     if (n == 0) return launch_matmul_generic(a, w, w_dtype, bias, out, out_dtype, rows, K, N, act, flags, s);
@@ -157,6 +170,11 @@ int32_t ttb_matmul(const void *a, int32_t a_dtype, const void *w, int32_t w_dtyp
 int32_t ttb_bmm(const void *a, int32_t a_dtype, const void *w, int32_t w_dtype, void *out, int32_t out_dtype, int64_t batch, int64_t M,
                 int64_t K, int64_t N, void *stream) {
     if (int32_t rc = validate(a, a_dtype, w, w_dtype, out, out_dtype, batch, M, K, N, TTB_ACT_NONE)) return rc;
+    if (w_dtype == TTB_BFLOAT16 && bf16_on_tensor_cores(out_dtype, K) && M / 32 <= 65535 && batch <= 65535) {
+        int *status = nullptr;
+        if (int32_t rc = status_word_address(&status)) return rc;
+        return launch_matmul_bf16(a, w, nullptr, out, out_dtype, batch, M, K, N, TTB_ACT_NONE, 0, status, (cudaStream_t)stream);
+    }
     return launch_bmm_generic(a, w, w_dtype, out, out_dtype, batch, M, K, N, (cudaStream_t)stream);
 }
 

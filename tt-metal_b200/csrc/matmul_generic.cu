@@ -1,8 +1,8 @@
 // Shape-generic matmul on the CUDA cores: any M, K, N that are multiples of 32, every supported
 // weight dtype. One 256-thread block owns a 32x32 output tile and walks K one tile at a time,
 // expanding block-float weight tiles to fp32 in shared memory. It is the correctness anchor for the
-// tensor-core kernels (same operands, same fp32 accumulation) and serves shapes their tiling does
-// not cover; it is not meant to be fast.
+// tensor-core kernels (same operands, same fp32 accumulation) and serves what they do not cover
+// (batched block-float operands, fp32 results of very short sums); it is not meant to be fast.
 #include "epilogue.cuh"
 
 namespace ttb {

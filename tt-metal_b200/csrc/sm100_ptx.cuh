@@ -178,6 +178,14 @@ __device__ __forceinline__ uint64_t smem_desc_sw32(uint32_t addr, uint32_t sbo) 
     return (uint64_t)((addr >> 4) & 0x3fffu) | (1ull << 16) | ((uint64_t)((sbo >> 4) & 0x3fffu) << 32) | (1ull << 46) | (6ull << 61);
 }
 
+// The same for an operand that is contiguous along M/N: rows of 32 bytes hold 16 consecutive M/N values of one K, eight K
+// rows form the 256-byte atom. `group` = bytes between neighbouring groups of 16 M/N values, `sbo` = bytes between groups of
+// eight K rows.
+__device__ __forceinline__ uint64_t smem_desc_sw32_mn(uint32_t addr, uint32_t group, uint32_t sbo) {
+    return (uint64_t)((addr >> 4) & 0x3fffu) | ((uint64_t)((group >> 4) & 0x3fffu) << 16) | ((uint64_t)((sbo >> 4) & 0x3fffu) << 32) | (1ull << 46) |
+           (6ull << 61);
+}
+
 // Instruction descriptor for kind::f16 with bf16 operands and an fp32 accumulator.
 // Bits: [4,6) D format (1 = f32), [7,10) A format (1 = bf16), [10,13) B format, 15 A major
 // (1 = M/N-contiguous), 16 B major, [17,23) N>>3, [24,29) M>>4.
