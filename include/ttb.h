@@ -178,7 +178,9 @@ int64_t ttb_matmul_workspace_bytes(int32_t w_dtype, int64_t batch, int64_t M, in
  * for a decode kernel - for as many launches as `out` has room for (out_len >= 5). Decode kernels take up to 256 rows and
  * any N that is a multiple of 32 (blocks of two tile rows when the row count is a multiple of 64 and N a multiple of 128,
  * else of one); the prefill kernel multiples of 128 rows from 512 up with N a multiple of 128; other row counts are served
- * as two ranges, and large row counts with an N the prefill kernel does not take as up to 16 decode launches of 256 rows. */
+ * as two ranges, and large row counts with an N the prefill kernel does not take as up to 16 decode launches of 256 rows.
+ * This is the plan of fp32 results. bf16 results of 64 rows and more are mostly computed by one kernel for any row and column
+ * count instead (csrc/matmul_rows.cu, which needs no workspace; the rule is rows_kernel_takes in csrc/matmul.cu). */
 int32_t ttb_matmul_plan(int32_t w_dtype, int64_t batch, int64_t M, int64_t K, int64_t N, int32_t flags, int64_t *out, int32_t out_len);
 int32_t ttb_matmul(const void *a_dev, int32_t a_dtype, const void *w_dev, int32_t w_dtype, const void *bias_dev,
                    void *out_dev, int32_t out_dtype, int64_t batch, int64_t M, int64_t K, int64_t N,

@@ -1,0 +1,76 @@
+"""Middling row counts of block-float weights (csrc/matmul_rows.cu) at the edges of its tiling, against 64-bit torch.
+
+Tolerance, per element: one rounding to bfloat16 (2^-9 of the result, doubled for the activations) and 2^-15 of sum |x||w|: at most
+K / 16 = 256 additions of 16 products in a row, each cutting off at most 2^-23 of the magnitudes added."""
+import pytest
+
+import cabi
+
+pytestmark = pytest.mark.gpu
+
+# rows, K, N: one tile row more than the decode kernels' blocks; a K range of fewer than four blocks and of one more than a group;
+# unequal row chunks; a partial column tile; clusters of 8, 3 and 2 blocks; whole rounds of tiles with a remainder launch, and more
+# tiles than SMs without one
+SHAPES = [(96, 32, 32), (96, 160, 96), (64, 4096, 128), (352, 992, 672), (544, 1056, 608), (224, 288, 4672), (1056, 512, 4672), (416, 96, 7168)]
+
+
+def reference(x, w, bias, act):
+    import torch
+    y, mag = x.double() @ w.double(), x.double().abs() @ w.double().abs()
+    if bias is not None:
+        y, mag = y + bias.double(), mag + bias.double().abs()
+    return {cabi.ACT_NONE: lambda v: v, cabi.ACT_RELU: torch.relu, cabi.ACT_GELU: torch.nn.functional.gelu, cabi.ACT_SILU: torch.nn.functional.silu}[act](y), mag
+
+
+def close(y, want, mag):
+    bound = 2.0 ** -8 * want.abs() + 2.0 ** -15 * mag
+    assert bool(((y.double() - want).abs() <= bound).all()), float(((y.double() - want).abs() / bound).max())
+
+
+def weight(ttb, fmt, K, N, scale, seed):
+    """Packed by the (bit-exact, separately tested) device packer, and the values it stands for."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    packed = ttb.pack(torch.randn(K, N, generator=g, device="cuda") * scale, fmt, 1, K, N)
+    return packed, ttb.unpack(packed, fmt, 1, K, N).reshape(K, N)
+
+
+@pytest.mark.parametrize("fmt", [cabi.BFLOAT8_B, cabi.BFLOAT4_B])
+@pytest.mark.parametrize("M,K,N", SHAPES)
+def test_against_64_bits(ttb, fmt, M, K, N):
+    import torch
+    for scale, act, with_bias, flags in ((0.02, cabi.ACT_NONE, False, 0), (3.0, cabi.ACT_GELU, True, 0), (0.02, cabi.ACT_SILU, True, cabi.MM_A_ROW_MAJOR | cabi.MM_OUT_ROW_MAJOR),
+                                         (0.02, cabi.ACT_RELU, False, cabi.MM_WEIGHTS_RESIDENT)):
+        packed, values = weight(ttb, fmt, K, N, scale, 3)   # (3.0: exponents above 127)
+        x = torch.randn(M, K, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda").bfloat16()
+        bias = torch.randn(1, N, device="cuda").bfloat16() if with_bias else None
+        bt = ttb.tilize(torch.cat([bias, bias.new_zeros(31, N)]), 1, 32, N) if with_bias else None
+        a = x.reshape(-1).contiguous() if flags & cabi.MM_A_ROW_MAJOR else ttb.tilize(x, 1, M, K)
+        buf = torch.full((8 + M * N + 512,), 7.0, dtype=torch.bfloat16, device="cuda")   # 16-byte aligned, a guard on both sides
+        out = buf[8:8 + M * N]
+        nbytes = ttb.matmul_workspace_bytes(fmt, 1, M, K, N, flags)
+        ws = torch.zeros(max(nbytes, 16), dtype=torch.uint8, device="cuda")
+        ttb.check(ttb.cdll.ttb_matmul(a.data_ptr(), cabi.BFLOAT16, packed.data_ptr(), fmt, bt.data_ptr() if with_bias else None, out.data_ptr(), cabi.BFLOAT16,
+                                      1, M, K, N, act, flags | cabi.MM_WORKSPACE_ZEROED, ws.data_ptr(), nbytes, None))
+        ttb.check(ttb.check_status(None))
+        assert bool((buf[:8] == 7.0).all()) and bool((buf[8 + M * N:] == 7.0).all()) and int(ws.count_nonzero()) == 0
+        y = out.reshape(M, N) if flags & cabi.MM_OUT_ROW_MAJOR else ttb.untilize(out.clone(), 1, M, N).reshape(M, N)
+        close(y, *reference(x, values, bias, act))
+
+
+def test_launches_that_follow_each_other_give_the_same_bytes(ttb):
+    """Overlapped launches (resident weights), each reading what the one before wrote; twice."""
+    import torch
+    M, K, fmt = 352, 1024, cabi.BFLOAT8_B
+    packed, _ = weight(ttb, fmt, K, K, 0.03, 9)
+    x = ttb.tilize(torch.randn(M, K, device="cuda").bfloat16(), 1, M, K)
+    results = []
+    for _ in range(2):
+        cur, outs = x, [torch.empty(M * K, dtype=torch.bfloat16, device="cuda") for _ in range(20)]
+        for o in outs:
+            ttb.check(ttb.cdll.ttb_matmul(cur.data_ptr(), cabi.BFLOAT16, packed.data_ptr(), fmt, None, o.data_ptr(), cabi.BFLOAT16, 1, M, K, K, 0,
+                                          cabi.MM_WEIGHTS_RESIDENT, None, 0, None))
+            cur = o
+        ttb.check(ttb.check_status(None))
+        results.append(outs)
+    assert all(torch.equal(a, b) for a, b in zip(*results)) and bool(torch.isfinite(results[0][-1].float()).all())

@@ -15,6 +15,7 @@ constexpr int kMaxSequenceStages = 4;   // stages (ttb_matmul_multi calls) one l
 struct alignas(64) WeightMaps {
     CUtensorMap m[TTB_MAX_GROUP];
 };
+int32_t make_weight_map(const uint8_t *w, int64_t K, int64_t N, int fmt, int group, CUtensorMap &map);
 int32_t make_weight_maps(const DecodeArgs &p, int fmt, WeightMaps &maps, int group = 3);
 // The activation [rows, K] (tiled or row-major bf16) as a tensor map whose box is three K blocks of 32 rows, delivered in
 // the MMA's K-major operand layout (`group` K blocks of 32 rows) with the 32-byte swizzle: [K block][16-column half][row][16 values].

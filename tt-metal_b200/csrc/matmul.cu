@@ -23,6 +23,8 @@ int64_t prefill_workspace_bytes(int64_t rows, int64_t K);
 int32_t launch_matmul_prefill(const void *a, const void *w, int w_dtype, const void *bias, void *out, int out_dtype, int64_t rows,
                               int64_t K, int64_t N, int act, int flags, void *workspace, int64_t workspace_bytes, int *status,
                               cudaStream_t stream);
+int32_t launch_matmul_rows(const void *a, const void *w, int w_dtype, const void *bias, void *out, int out_dtype, int64_t rows, int64_t K, int64_t N,
+                              int act, int flags, int *status, cudaStream_t stream);
 
 namespace {
 
@@ -59,6 +61,21 @@ int32_t validate(const void *a, int a_dtype, const void *w, int w_dtype, void *o
 // cut off low bits) come out further from 64 bits than a chain of fused multiply-adds (2-norm at K = 64: 6.5e-8 against
 // 5.1e-8; at 128: 7.1e-8 against 7.3e-8, and the longer the further ahead).
 bool bf16_on_tensor_cores(int out_dtype, int64_t K) { return out_dtype == TTB_BFLOAT16 || K >= 128; }
+
+// bfloat16 results that the kernel of matmul_rows.cu takes, whole and whatever the column count (fp32 results keep the row ranges
+// below, whose shorter chains of additions bring them closer to 64 bits). Three lines, with both sides measured (us):
+//  * 96 rows and more: 96 x 4096 x 4096 17.0 with the decode kernel, 13.2 here; 128 x 4096 x 14336 bfloat4_b 46.2 / 28.4;
+//  * 64 rows while its 128-column tiles number at most half the SMs and their K range can be shared: 64 x 8192 x 8192 35.7 /
+//    27.2, 64 x 4096 x 1024 14.9 / 8.9, but 64 x 4096 x 14336 (112 tiles) 21.1 / 26.2;
+//  * not where the prefill kernel's 256 x 256 blocks fill three quarters of a round: 2048 x 8192 x 28672 864 there, 948 here,
+//    1024 x 2048 x 8192 48.3 / 52.9; below that 512 x 4096 x 4096 (32 blocks) 74.8 / 24.0.
+bool rows_kernel_takes(int w_dtype, int out_dtype, int64_t rows, int64_t K, int64_t N, int flags) {
+    if (w_dtype == TTB_BFLOAT16 || out_dtype != TTB_BFLOAT16 || (flags & (TTB_MM_FORCE_GENERIC | TTB_MM_DECODE_SMEM_OPERAND))) return false;
+    constexpr int64_t kSms = 148;
+    if (rows == 64) return (N + 127) / 128 * 2 <= kSms;
+    if (rows < 96) return false;
+    return !(prefill_supported(w_dtype, rows, K, N) && rows * N / 65536 * 4 >= kSms * 3);
+}
 
 // Row ranges of one matmul and the tensor-core kernel that takes each: the decode kernels serve up to 256 rows, the prefill
 // kernel multiples of 128 from 512 up (column counts that are multiples of 128). Row counts in between run as two decode
@@ -121,8 +138,7 @@ int64_t ttb_matmul_workspace_bytes(int32_t w_dtype, int64_t batch, int64_t M, in
 }
 
 /* Which block-float kernels ttb_matmul would use: out[0] = launches (0: none of them - the shape-generic CUDA-core kernel, or for
- * bfloat16 weights usually the kernel of matmul_bf16.cu), then per launch its rows
- * and 1 for the prefill kernel, 0 for a decode kernel - for as many launches as `out` has room for (at least two). */
+ * bfloat16 weights usually the kernel of matmul_bf16.cu; fp32 results, see rows_kernel_takes), then per launch its rows and 1 for the prefill kernel, 0 for a decode kernel - for as many launches as `out` has room for (at least two). */
 int32_t ttb_matmul_plan(int32_t w_dtype, int64_t batch, int64_t M, int64_t K, int64_t N, int32_t flags, int64_t *out, int32_t out_len) {
     if (!out || out_len < 5) return fail(TTB_E_INVALID, "ttb_matmul_plan: needs room for 5 values");
     RowChunk chunks[kMaxRowChunks];
@@ -145,6 +161,11 @@ int32_t ttb_matmul(const void *a, int32_t a_dtype, const void *w, int32_t w_dtyp
         int *status = nullptr;
         if (int32_t rc = status_word_address(&status)) return rc;
         return launch_matmul_bf16(a, w, bias, out, out_dtype, 1, rows, K, N, act, flags, status, s);
+    }
+    if (rows_kernel_takes(w_dtype, out_dtype, rows, K, N, flags)) {
+        int *status = nullptr;
+        if (int32_t rc = status_word_address(&status)) return rc;
+        return launch_matmul_rows(a, w, w_dtype, bias, out, out_dtype, rows, K, N, act, flags, status, s);
     }
     RowChunk chunks[kMaxRowChunks];
     const int n = (flags & TTB_MM_FORCE_GENERIC) ? 0 : plan_rows(w_dtype, rows, K, N, chunks);

@@ -65,12 +65,6 @@ struct Args {
     int *status;
 };
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-// One arrival of this thread on the barrier (part of its count) once all its earlier cp.async have landed.
-__device__ __forceinline__ void cp_async_arrive(uint32_t bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -189,9 +183,8 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_bf16_kernel(const __grid_c
         // ---------------- producers ----------------
         grid_dep_wait();
         const int pw = warp - kEpiWarps;
-        // inside a face: lane l takes 16-byte chunk l; the halves of rows 4..7 of every eight are exchanged (address bit 4 ^= bit 7)
-        const int fr = lane >> 1, fh = lane & 1;
-        const uint32_t face_dst = (uint32_t)((lane * 16) ^ ((lane & 8) << 1));
+        const int fr = lane >> 1, fh = lane & 1;   // inside a face: lane l takes 16-byte chunk l
+        const uint32_t face_dst = face_chunk_sw32(lane);
         int s = 0;
         uint32_t ph = 0;
         bool ok = true;

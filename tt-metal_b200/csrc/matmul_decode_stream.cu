@@ -600,9 +600,9 @@ int32_t launch_one(const DecodeArgs &p, const WeightMaps &maps, bool overlap, cu
 }  // namespace
 
 
-// Tensor maps of the launch's weights. cuTensorMapEncodeTiled is reached through the runtime's driver entry point (no link
-// against the driver library).
-int32_t make_weight_maps(const DecodeArgs &p, int fmt, WeightMaps &maps, int group) {
+// A packed weight [K, N] as a tensor map: [K blocks][tiles per row][tile as 8-byte words], box of `group` K blocks x four tiles.
+// cuTensorMapEncodeTiled is reached through the runtime's driver entry point (no link against the driver library).
+int32_t make_weight_map(const uint8_t *w, int64_t K, int64_t N, int fmt, int group, CUtensorMap &map) {
     using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -614,18 +614,21 @@ int32_t make_weight_maps(const DecodeArgs &p, int fmt, WeightMaps &maps, int gro
         if (!fn || qres != cudaDriverEntryPointSuccess) return fail(TTB_E_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
         encode = reinterpret_cast<EncodeFn>(fn);
     }
-    const cuuint64_t tile_bytes = (cuuint64_t)bfp_tile_bytes(fmt);
-    for (int j = 0; j < p.nprob; ++j) {
-        const cuuint64_t Nt = (cuuint64_t)(p.Nv[j] / 32), Kt = (cuuint64_t)p.Kt;
-        const cuuint64_t dims[3] = {tile_bytes / 8, Nt, Kt};
-        const cuuint64_t strides[2] = {tile_bytes, Nt * tile_bytes};
-        const cuuint32_t box[3] = {(cuuint32_t)(tile_bytes / 8), 4, (cuuint32_t)group};   // `group` K blocks = one group of stages
-        const cuuint32_t estr[3] = {1, 1, 1};
-        const CUresult r = encode(&maps.m[j], CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<uint8_t *>(p.wv[j]), dims, strides, box, estr,
-                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return fail(TTB_E_CUDA, "cuTensorMapEncodeTiled failed with %d for weight %d", (int)r, j);
-    }
+    const cuuint64_t tile_bytes = (cuuint64_t)bfp_tile_bytes(fmt), Nt = (cuuint64_t)(N / 32), Kt = (cuuint64_t)(K / 32);
+    const cuuint64_t dims[3] = {tile_bytes / 8, Nt, Kt};
+    const cuuint64_t strides[2] = {tile_bytes, Nt * tile_bytes};
+    const cuuint32_t box[3] = {(cuuint32_t)(tile_bytes / 8), 4, (cuuint32_t)group};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<uint8_t *>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(TTB_E_CUDA, "cuTensorMapEncodeTiled failed with %d for a weight", (int)r);
+    return TTB_OK;
+}
+
+// Tensor maps of the launch's weights.
+int32_t make_weight_maps(const DecodeArgs &p, int fmt, WeightMaps &maps, int group) {
+    for (int j = 0; j < p.nprob; ++j)
+        if (int32_t rc = make_weight_map(p.wv[j], p.K, p.Nv[j], fmt, group, maps.m[j])) return rc;
     for (int j = p.nprob; j < TTB_MAX_GROUP; ++j) maps.m[j] = maps.m[0];
     return TTB_OK;
 }

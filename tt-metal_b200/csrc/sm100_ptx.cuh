@@ -138,15 +138,31 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst_smem, const void *tenso
         "l"(tensor_map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
         : "memory");
 }
+// The same without a cache hint (data that other blocks will read again from L2).
 __device__ __forceinline__ void tma_load_3d_plain(uint32_t dst_smem, const void *tensor_map, int x, int y, int z, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst_smem),
         "l"(tensor_map), "r"(x), "r"(y), "r"(z), "r"(bar)
         : "memory");
 }
+
 // Makes writes of other GPUs (or of earlier kernels) that this thread has observed through generic loads visible to the
 // asynchronous proxy, i.e. to tensor-map copies this thread issues afterwards.
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+
+// ---- 16-byte asynchronous copies by ordinary threads (generic proxy) -----------------------------
+__device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src_gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src_gmem) : "memory");
+}
+// One arrival of this thread on the barrier (part of its count) once all its earlier cp.async have landed. Whoever waits for
+// them and then hands the data to the tensor cores orders the two with fence_proxy_async_smem(): a fence in the copying
+// thread would wait for its later copies as well.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Where lane `lane` puts 16-byte chunk `lane` of a 16x16 bf16 face (512 contiguous bytes, rows of 32) so that the face is in
+// the 32-byte-swizzled operand layout: the halves of rows 4..7 of every eight change places (address bit 4 ^= bit 7).
+__device__ __forceinline__ uint32_t face_chunk_sw32(int lane) { return (uint32_t)((lane * 16) ^ ((lane & 8) << 1)); }
 
 // ---- tensor memory -------------------------------------------------------------------------------
 // Whole-warp calls. `ncols` is a power of two in [32, 512].
