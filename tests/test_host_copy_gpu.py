@@ -1,0 +1,49 @@
+"""Copies of pageable host memory through the pinned staging buffers (csrc/host_copy.cu): sizes around the chunk and the threshold,
+unaligned host addresses, several threads at once, pinned memory - the same bytes."""
+import threading
+
+import pytest
+
+import cabi
+
+pytestmark = pytest.mark.gpu
+MB = 1 << 20
+
+
+def round_trip(ttb, bytes_, skip, pinned=False):
+    import torch
+    src = torch.randint(0, 256, (bytes_ + skip,), dtype=torch.uint8)
+    dst = torch.zeros(bytes_ + skip + 64, dtype=torch.uint8)
+    if pinned:
+        src, dst = src.pin_memory(), dst.pin_memory()
+    dev = torch.empty(bytes_, dtype=torch.uint8, device="cuda")
+    ttb.check(ttb.cdll.ttb_memcpy_h2d(dev.data_ptr(), src.data_ptr() + skip, bytes_, None))
+    ttb.check(ttb.cdll.ttb_memcpy_d2h(dst.data_ptr() + skip, dev.data_ptr(), bytes_, None))
+    ttb.check(ttb.cdll.ttb_stream_synchronize(None))
+    assert torch.equal(dst[skip:skip + bytes_], src[skip:]) and not dst[:skip].any() and not dst[skip + bytes_:].any()
+
+
+@pytest.mark.parametrize("bytes_,skip", [(4 * MB - 1, 0), (4 * MB, 0), (4 * MB + 1, 3), (5 * MB, 1), (16 * MB, 0), (16 * MB + 12345, 7), (40 * MB - 5, 0)])
+def test_round_trip(ttb, bytes_, skip):
+    round_trip(ttb, bytes_, skip)
+    round_trip(ttb, bytes_, skip, pinned=True)
+
+
+def test_several_threads(ttb):
+    failures = []
+
+    def work(n):
+        try:
+            import torch
+            torch.cuda.set_device(0)
+            for _ in range(3):
+                round_trip(ttb, 9 * MB + n, n)
+        except BaseException as e:   # noqa: BLE001
+            failures.append(e)
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures

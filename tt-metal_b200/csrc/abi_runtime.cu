@@ -6,6 +6,7 @@
 #include "common.cuh"
 
 namespace ttb {
+bool copy_staged(void *dev, void *host, size_t bytes, bool to_device, cudaStream_t stream, cudaError_t &error);
 static thread_local char g_err[512] = "";
 
 int32_t fail(int32_t code, const char *fmt, ...) {
@@ -17,6 +18,7 @@ int32_t fail(int32_t code, const char *fmt, ...) {
 }
 }  // namespace ttb
 
+using ttb::copy_staged;
 using ttb::fail;
 
 extern "C" {
@@ -96,12 +98,22 @@ int32_t ttb_host_free(void *host_ptr) {
 int32_t ttb_memcpy_h2d(void *dst, const void *src, size_t bytes, void *stream) {
     if (bytes == 0) return TTB_OK;
     if (!dst || !src) return fail(TTB_E_INVALID, "ttb_memcpy_h2d: null pointer");
+    cudaError_t staged;
+    if (copy_staged(dst, const_cast<void *>(src), bytes, /*to_device=*/true, (cudaStream_t)stream, staged)) {
+        TTB_CUDA_TRY(staged);
+        return TTB_OK;
+    }
     TTB_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, (cudaStream_t)stream));
     return TTB_OK;
 }
 int32_t ttb_memcpy_d2h(void *dst, const void *src, size_t bytes, void *stream) {
     if (bytes == 0) return TTB_OK;
     if (!dst || !src) return fail(TTB_E_INVALID, "ttb_memcpy_d2h: null pointer");
+    cudaError_t staged;
+    if (copy_staged(const_cast<void *>(src), dst, bytes, /*to_device=*/false, (cudaStream_t)stream, staged)) {
+        TTB_CUDA_TRY(staged);
+        return TTB_OK;
+    }
     TTB_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     return TTB_OK;
 }
