@@ -58,6 +58,29 @@ def test_against_64_bits(ttb, fmt, M, K, N):
         close(y, *reference(x, values, bias, act))
 
 
+@pytest.mark.parametrize("fmt", [cabi.BFLOAT8_B, cabi.BFLOAT4_B])
+@pytest.mark.parametrize("M,K,Ns", [(96, 512, (512, 96, 160)), (128, 1024, (1024, 128)), (256, 288, (96, 4672, 32, 4096))])
+def test_several_weights_in_one_launch(ttb, fmt, M, K, Ns):
+    import ctypes
+    import torch
+    x = torch.randn(M, K, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda").bfloat16()
+    a, n = ttb.tilize(x, 1, M, K), len(Ns)
+    ws = [weight(ttb, fmt, K, N, 0.02, 20 + j) for j, N in enumerate(Ns)]
+    biases = [torch.randn(1, N, device="cuda").bfloat16() if j != 1 else None for j, N in enumerate(Ns)]
+    tiled = [ttb.tilize(torch.cat([b, b.new_zeros(31, N)]), 1, 32, N) if b is not None else None for b, N in zip(biases, Ns)]
+    outs = [torch.full((M * N + 64,), 7.0, dtype=torch.bfloat16, device="cuda") for N in Ns]
+    ptrs = lambda ts: (ctypes.c_void_p * n)(*[t.data_ptr() if t is not None else None for t in ts])   # noqa: E731
+    arr_n = (ctypes.c_int64 * n)(*Ns)
+    nbytes = ttb.matmul_multi_workspace_bytes(fmt, 1, M, K, n, arr_n)
+    wsp = torch.zeros(max(nbytes, 16), dtype=torch.uint8, device="cuda")
+    ttb.check(ttb.cdll.ttb_matmul_multi(a.data_ptr(), cabi.BFLOAT16, n, ptrs([p for p, _ in ws]), fmt, ptrs(tiled), ptrs(outs), cabi.BFLOAT16, 1, M, K, arr_n,
+                                        cabi.ACT_SILU, cabi.MM_WORKSPACE_ZEROED | cabi.MM_WEIGHTS_RESIDENT, wsp.data_ptr(), nbytes, None, None, None))
+    ttb.check(ttb.check_status(None))
+    for (_, values), b, o, N in zip(ws, biases, outs, Ns):
+        assert bool((o[M * N:] == 7.0).all())
+        close(ttb.untilize(o[:M * N].clone(), 1, M, N).reshape(M, N), *reference(x, values, b, cabi.ACT_SILU))
+
+
 def test_launches_that_follow_each_other_give_the_same_bytes(ttb):
     """Overlapped launches (resident weights), each reading what the one before wrote; twice."""
     import torch

@@ -22,6 +22,8 @@ static constexpr int64_t kCounterBytes = 65536;
 static constexpr int64_t kAccumBytes = 16 << 20;
 
 int32_t launch_decode_tmem(const DecodeArgs *stages, int n, int fmt, int nb, int *sync, bool overlap, cudaStream_t stream);
+int32_t launch_matmul_rows(const void *a, int count, const void *const *w, int w_dtype, const void *const *bias, void *const *out, int out_dtype, int64_t rows,
+                           int64_t K, const int64_t *N, int act, int flags, int *status, cudaStream_t stream);
 // The tail of the counter region belongs to the launch as a whole (matmul_decode_tmem.cu: blocks that have finished, tiles
 // each stage has stored); the per-tile counters stay below it.
 static constexpr int kSyncInts = 16;
@@ -540,6 +542,14 @@ extern "C" int32_t ttb_matmul_multi(const void *a, int32_t a_dtype, int32_t coun
     if (batch <= 0 || M <= 0 || M % 32) return fail(TTB_E_INVALID, "ttb_matmul_multi: batch, M, K must be positive and M, K multiples of 32");
     const int64_t rows = batch * M;
     if (int32_t rc = validate_multi("ttb_matmul_multi", a, a_dtype, count, w, w_dtype, out, out_dtype, rows, K, N, act, flags, gather, wait)) return rc;
+    // bfloat16 results of 96 rows and more, of one rank and not gated: the kernel that expands a weight once for all its rows (us
+    // before / now: 96 x 4096 x [4096, 1024, 1024] 19.5 / 18.5, 128 rows 21.5 / 18.6, 256 rows 39.9 / 24.6, 128 x 8192 x [28672,
+    // 28672] 270 / 155).
+    if (rows >= 96 && out_dtype == TTB_BFLOAT16 && !gather && !wait && !(flags & (TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_GATED))) {
+        int *status = nullptr;
+        if (int32_t rc = status_word_address(&status)) return rc;
+        return launch_matmul_rows(a, count, w, w_dtype, bias, out, out_dtype, rows, K, N, act, flags, status, (cudaStream_t)stream);
+    }
     return launch_matmul_decode_multi(a, count, w, w_dtype, bias, out, out_dtype, rows, K, N, act,
                                       flags & (TTB_MM_A_ROW_MAJOR | TTB_MM_OUT_ROW_MAJOR | TTB_MM_DETERMINISTIC | TTB_MM_WEIGHTS_RESIDENT | TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_GATED),
                                       workspace, workspace_bytes, (flags & TTB_MM_WORKSPACE_ZEROED) != 0, /*compact=*/false,

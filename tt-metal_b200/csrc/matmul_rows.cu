@@ -1,5 +1,5 @@
 // Matmul for middling row counts (large decode batches, short prompts; any size above that the prefill kernel does not take):
-// out[rows, N] = act(a[rows, K] x W[K, N] + bias) with W in packed bfloat8_b / bfloat4_b tiles; rows, K and N multiples of 32.
+// out_j[rows, N_j] = act(a[rows, K] x W_j[K, N_j] + bias_j) for up to four weights W_j that share the activation, in packed bfloat8_b / bfloat4_b tiles; rows, K and N multiples of 32.
 //
 // "Swap-AB", as in the decode kernels: the MMA's M dimension (128 TMEM lanes) runs over weight columns, its N dimension over up
 // to 256 activation rows, and a block owns 128 columns x one chunk of rows, so that a weight is expanded once per chunk (the
@@ -65,10 +65,14 @@ struct Layout {
 };
 
 struct alignas(64) Args {
-    CUtensorMap wmap;       // the packed weight as [K blocks][tiles per row][tile as 8-byte words], box of kGroup x 4 tiles
-    const uint16_t *a, *bias;
-    void *out;
-    int64_t rows, K, N;
+    // up to four weights that share the activation; their column tiles form one list, weight j's from tstart[j]
+    CUtensorMap wmap[TTB_MAX_GROUP];   // packed weights as [K blocks][tiles per row][tile as 8-byte words], box of kGroup x 4 tiles
+    const uint16_t *bias[TTB_MAX_GROUP];
+    void *out[TTB_MAX_GROUP];
+    int64_t N[TTB_MAX_GROUP];
+    int weights, tstart[TTB_MAX_GROUP + 1];
+    const uint16_t *a;
+    int64_t rows, K;
     int Kt;                 // K blocks
     int chunks, chunk_rows; // row chunks and rows of each (the last may have fewer)
     int tile0, tiles;       // this launch's tiles: tile0 .. tile0 + tiles - 1; row chunks vary fastest
@@ -95,25 +99,25 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t local_addr, uint32_t
 
 // Four neighbouring columns n .. n + 3 of one row: bias, activation, store.
 template <int ACT>
-__device__ __forceinline__ void finish4(const Args &p, int64_t row, int64_t n, float4 v, float4 b) {
+__device__ __forceinline__ void finish4(const Args &p, int w, int64_t row, int64_t n, float4 v, float4 b) {
     v.x = apply_activation_t<ACT>(v.x + b.x); v.y = apply_activation_t<ACT>(v.y + b.y);
     v.z = apply_activation_t<ACT>(v.z + b.z); v.w = apply_activation_t<ACT>(v.w + b.w);
-    const int64_t off = p.out_row_major ? row * p.N + n : tiled_offset(row, n, p.N >> 5);
+    const int64_t off = p.out_row_major ? row * p.N[w] + n : tiled_offset(row, n, p.N[w] >> 5);
     if (p.out_dtype == TTB_FLOAT32)
-        *reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.out) + off) = v;
+        *reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.out[w]) + off) = v;
     else
-        *reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(p.out) + off) =
+        *reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(p.out[w]) + off) =
             make_uint2((uint32_t)f32_to_bf16_bits(v.x) | ((uint32_t)f32_to_bf16_bits(v.y) << 16),
                        (uint32_t)f32_to_bf16_bits(v.z) | ((uint32_t)f32_to_bf16_bits(v.w) << 16));
 }
-__device__ __forceinline__ float4 bias4(const Args &p, int64_t n) {
-    if (!p.bias || n >= p.N) return make_float4(0.f, 0.f, 0.f, 0.f);
-    return make_float4(bias_at(p.bias, n), bias_at(p.bias, n + 1), bias_at(p.bias, n + 2), bias_at(p.bias, n + 3));
+__device__ __forceinline__ float4 bias4(const Args &p, int w, int64_t n) {
+    if (!p.bias[w] || n >= p.N[w]) return make_float4(0.f, 0.f, 0.f, 0.f);
+    return make_float4(bias_at(p.bias[w], n), bias_at(p.bias[w], n + 1), bias_at(p.bias[w], n + 2), bias_at(p.bias[w], n + 3));
 }
 // Rows r0, r0 + step, ... < r1 of a [rows][BN] fp32 slab in shared memory: a warp's lanes take four columns each.
 template <int ACT>
-__device__ __forceinline__ void finish_rows(const Args &p, uint32_t slab, int r0, int r1, int step, int64_t row_base, int64_t n, int blocks, const float4 b) {
-    if (n >= p.N) return;
+__device__ __forceinline__ void finish_rows(const Args &p, int w, uint32_t slab, int r0, int r1, int step, int64_t row_base, int64_t n, int blocks, const float4 b) {
+    if (n >= p.N[w]) return;
     for (int r = r0; r < r1; r += step) {
         const uint32_t at = slab + (uint32_t)(r * BN * 4) + (uint32_t)((threadIdx.x & 31) * 16);
         float4 v;
@@ -126,7 +130,7 @@ __device__ __forceinline__ void finish_rows(const Args &p, uint32_t slab, int r0
                 v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
             }
         }
-        finish4<ACT>(p, row_base + r, n, v, b);
+        finish4<ACT>(p, w, row_base + r, n, v, b);
     }
 }
 
@@ -177,7 +181,14 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
     const int kb0 = (int)((int64_t)p.Kt * rank / p.split), kb1 = (int)((int64_t)p.Kt * (rank + 1) / p.split);
     const int first = (int)blockIdx.x / p.split, step = (int)gridDim.x / p.split;
     auto chunk_of = [&](int t) { return (p.tile0 + t) % p.chunks; };
-    auto column_tile_of = [&](int t) { return (p.tile0 + t) / p.chunks; };
+    auto column_tile_of = [&](int t, int &w) {   // the weight, and the column tile inside it
+        const int c = (p.tile0 + t) / p.chunks;
+        w = 0;
+#pragma unroll
+        for (int j = 1; j < TTB_MAX_GROUP; ++j)
+            if (j < p.weights && c >= p.tstart[j]) w = j;
+        return c - p.tstart[w];
+    };
     auto rows_of = [&](int chunk) { return (int)min((int64_t)p.chunk_rows, p.rows - (int64_t)chunk * p.chunk_rows); };
 
     if (warp < kExpandWarps) {
@@ -221,13 +232,14 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
         uint32_t ph = 0;
         bool ok = true;
         for (int t = first; ok && t < p.tiles; t += step) {
-            const int nt = column_tile_of(t);
+            int w;
+            const int nt = column_tile_of(t, w);
             for (int kb = kb0; kb < kb1; kb += kGroup) {
                 if (!__all_sync(0xffffffffu, mbar_wait(empty_p(s), ph ^ 1u, abort_flag, p.status, 53))) { ok = false; break; }
                 if (leader) {
                     // (always a whole box: what lies beyond the weight reads as zeros, a surplus K block is not expanded)
                     mbar_arrive_expect_tx(full_p(s), kGroup * L::kPStageBytes);
-                    tma_load_3d_plain(sbase + L::pk + s * kGroup * L::kPStageBytes, &p.wmap, 0, nt * 4, kb, full_p(s));
+                    tma_load_3d_plain(sbase + L::pk + s * kGroup * L::kPStageBytes, &p.wmap[w], 0, nt * 4, kb, full_p(s));
                 }
                 if (++s == kPRing) { s = 0; ph ^= 1u; }
             }
@@ -319,7 +331,8 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
         bool ok = true;
         for (int t = first; ok && t < p.tiles; t += step, ++n) {
             const int chunk = chunk_of(t), nrows = rows_of(chunk);
-            const int64_t row_base = (int64_t)chunk * p.chunk_rows, col0 = (int64_t)column_tile_of(t) * BN + lane * 4;
+            int w;
+            const int64_t row_base = (int64_t)chunk * p.chunk_rows, col0 = (int64_t)column_tile_of(t, w) * BN + lane * 4;
             // (the eight warps meet at named barriers below: they go on together or not at all)
             int good = mbar_wait(acc_full, (uint32_t)(n & 1), abort_flag, p.status, 57) ? 1 : 0;
             asm volatile(
@@ -329,7 +342,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
                 : "memory");
             if (!good) { ok = false; break; }
             tc_fence_after_sync();
-            const float4 b = bias4(p, col0);
+            const float4 b = bias4(p, w, col0);
             for (int r0 = 0; r0 < nrows; r0 += kStageRows) {
                 uint32_t v[16];
                 tmem_ld16(t_lane + (uint32_t)(r0 + half * 16), v);
@@ -344,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
                 }
                 if (p.split == 1) {
                     asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
-                    TTB_DISPATCH_ACT(p.act, finish_rows<ACT>(p, slab, ew, kStageRows, kEpiWarps, row_base + r0, col0, 1, b));
+                    TTB_DISPATCH_ACT(p.act, finish_rows<ACT>(p, w, slab, ew, kStageRows, kEpiWarps, row_base + r0, col0, 1, b));
                     asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
                 }
             }
@@ -357,9 +370,10 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
         cluster_sync();
         if (*abort_flag == 0) {
             const int chunk = chunk_of(first), nrows = rows_of(chunk);
-            const int64_t col0 = (int64_t)column_tile_of(first) * BN + lane * 4;
-            const float4 b = bias4(p, col0);
-            TTB_DISPATCH_ACT(p.act, finish_rows<ACT>(p, sbase + L::x, nrows * rank / p.split + warp, nrows * (rank + 1) / p.split, kThreads / 32,
+            int w;
+            const int64_t col0 = (int64_t)column_tile_of(first, w) * BN + lane * 4;
+            const float4 b = bias4(p, w, col0);
+            TTB_DISPATCH_ACT(p.act, finish_rows<ACT>(p, w, sbase + L::x, nrows * rank / p.split + warp, nrows * (rank + 1) / p.split, kThreads / 32,
                                                      (int64_t)chunk * p.chunk_rows, col0, p.split, b));
         }
         __syncwarp();
@@ -469,8 +483,9 @@ int32_t launch_fmt(Args &p, bool overlap, cudaStream_t stream) {
         return c;
     };
     // Row chunks: as few as possible, or up to twice as many where that fills the last round of blocks better. A K block takes
-    // about 125 ns + 0.48 ns per row of the chunk (fitted to timings of 64 to 256 rows), a further launch or exchange some 2 us.
-    const int tile_rows = (int)(p.rows / 32), least = (tile_rows + 7) / 8, nt = (int)((p.N + BN - 1) / BN);
+    // about 125 ns + 0.48 ns per row of the chunk, the exchange of partial sums 1 us + 16 ns per row, a further launch 1 us (fitted
+    // to timings of 64 to 256 rows: 256 x 2048 x 2048 as one chunk 13.0 us, as two 10.8; 512 x 4096 x 4096 as two 24.0, as four 27.7).
+    const int tile_rows = (int)(p.rows / 32), least = (tile_rows + 7) / 8, nt = p.tstart[p.weights];
     double best = 1e30;
     int split = 1;
     for (int c = least; c <= 2 * least && c <= tile_rows; ++c) {
@@ -478,7 +493,8 @@ int32_t launch_fmt(Args &p, bool overlap, cudaStream_t stream) {
         const int64_t t = (int64_t)chunks * nt, rest = t % d.sms;
         const int s = rest ? split_for((int)rest) : 1;
         const double kb = 125.0 + 0.48 * 32 * per;
-        const double cost = (double)(t / d.sms) * p.Kt * kb + (rest ? (p.Kt + s - 1) / s * kb + (s > 1 || t > d.sms ? 2000.0 : 0.0) : 0.0);
+        const double exchange = s > 1 ? 1000.0 + 16.0 * 32 * per : 0.0;
+        const double cost = (double)(t / d.sms) * p.Kt * kb + (rest ? (p.Kt + s - 1) / s * kb + exchange + (s > 1 && t > d.sms ? 1000.0 : 0.0) : 0.0);
         if (cost < best) {
             best = cost;
             split = s;
@@ -492,18 +508,28 @@ int32_t launch_fmt(Args &p, bool overlap, cudaStream_t stream) {
 }
 }  // namespace
 
-// The whole matmul in one or two launches, whatever the row and column counts.
-int32_t launch_matmul_rows(const void *a, const void *w, int w_dtype, const void *bias, void *out, int out_dtype, int64_t rows, int64_t K, int64_t N,
-                              int act, int flags, int *status, cudaStream_t stream) {
+// `count` matmuls that share the activation, in one or two launches, whatever the row and column counts.
+int32_t launch_matmul_rows(const void *a, int count, const void *const *w, int w_dtype, const void *const *bias, void *const *out, int out_dtype, int64_t rows,
+                           int64_t K, const int64_t *N, int act, int flags, int *status, cudaStream_t stream) {
     Args p = {};
-    p.a = (const uint16_t *)a; p.bias = (const uint16_t *)bias; p.out = out;
-    p.rows = rows; p.K = K; p.N = N; p.Kt = (int)(K / BK);
+    p.a = (const uint16_t *)a;
+    p.rows = rows; p.K = K; p.Kt = (int)(K / BK);
     p.act = act; p.out_dtype = out_dtype;
     p.a_row_major = (flags & TTB_MM_A_ROW_MAJOR) != 0;
     p.out_row_major = (flags & TTB_MM_OUT_ROW_MAJOR) != 0;
     p.status = status;
-    if (rows / 32 * ((N + BN - 1) / BN) > INT32_MAX / 8) return fail(TTB_E_UNSUPPORTED, "ttb_matmul: too many output tiles");
-    if (int32_t rc = make_weight_map((const uint8_t *)w, K, N, w_dtype, kGroup, p.wmap)) return rc;
+    p.weights = count;
+    int64_t tiles = 0;
+    for (int j = 0; j < count; ++j) {
+        p.bias[j] = (const uint16_t *)(bias ? bias[j] : nullptr);
+        p.out[j] = out[j];
+        p.N[j] = N[j];
+        p.tstart[j] = (int)tiles;
+        tiles += (N[j] + BN - 1) / BN;
+        if (rows / 32 * tiles > INT32_MAX / 8) return fail(TTB_E_UNSUPPORTED, "ttb_matmul: too many output tiles");
+        if (int32_t rc = make_weight_map((const uint8_t *)w[j], K, N[j], w_dtype, kGroup, p.wmap[j])) return rc;
+    }
+    p.tstart[count] = (int)tiles;
     const bool overlap = (flags & TTB_MM_WEIGHTS_RESIDENT) != 0;
     return w_dtype == TTB_BFLOAT8_B ? launch_fmt<TTB_BFLOAT8_B>(p, overlap, stream) : launch_fmt<TTB_BFLOAT4_B>(p, overlap, stream);
 }
