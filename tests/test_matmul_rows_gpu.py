@@ -10,8 +10,9 @@ pytestmark = pytest.mark.gpu
 
 # rows, K, N: one tile row more than the decode kernels' blocks; a K range of fewer than four blocks and of one more than a group;
 # unequal row chunks; a partial column tile; clusters of 8, 3 and 2 blocks; whole rounds of tiles with a remainder launch, and more
-# tiles than SMs without one
-SHAPES = [(96, 32, 32), (96, 160, 96), (64, 4096, 128), (352, 992, 672), (544, 1056, 608), (224, 288, 4672), (1056, 512, 4672), (416, 96, 7168)]
+# tiles than SMs without one; chunks of 256 rows
+SHAPES = [(96, 32, 32), (96, 160, 96), (64, 4096, 128), (352, 992, 672), (544, 1056, 608), (224, 288, 4672), (1056, 512, 4672), (416, 96, 7168),
+          (512, 4096, 4096)]
 
 
 def reference(x, w, bias, act):

@@ -66,15 +66,24 @@ bool bf16_on_tensor_cores(int out_dtype, int64_t K) { return out_dtype == TTB_BF
 // below, whose shorter chains of additions bring them closer to 64 bits). Three lines, with both sides measured (us):
 //  * 96 rows and more: 96 x 4096 x 4096 17.0 with the decode kernel, 13.2 here; 128 x 4096 x 14336 bfloat4_b 46.2 / 28.4;
 //  * 64 rows while its 128-column tiles number at most half the SMs and their K range can be shared: 64 x 8192 x 8192 35.7 /
-//    27.2, 64 x 4096 x 1024 14.9 / 8.9, but 64 x 4096 x 14336 (112 tiles) 21.1 / 26.2;
-//  * not where the prefill kernel's 256 x 256 blocks fill three quarters of a round: 2048 x 8192 x 28672 864 there, 948 here,
-//    1024 x 2048 x 8192 48.3 / 52.9; below that 512 x 4096 x 4096 (32 blocks) 74.8 / 24.0.
+//    27.2, 64 x 4096 x 1024 14.9 / 8.9, but 64 x 4096 x 14336 (112 tiles) 21.1 / 26.2, and a 64-row layer with a down projection of
+//    K = 21504 took 185 / 195;
+//  * where the prefill kernel applies, it keeps two kinds of shapes: bfloat8_b weights whose 256 x 256 blocks come to five or more
+//    whole rounds with little left over (2048 x 8192 x 28672, 6.05 rounds: 862 there, 890 here; broken rounds favour the finer
+//    tiles here: 1.7 rounds, 2048 x 8192 x 8192, 268 / 239; 3.5 rounds, 2048 x 2048 x 16384, 168 / 147; bfloat4_b 6.05 rounds 932 /
+//    835), and single, nearly full rounds of a short K range (1024 x 2048 x 8192 bfloat4_b 45.2 / 46.0, but 2048 x 4096 x 4096
+//    81.2 / 74.0); 512 x 4096 x 4096 (32 blocks) 74.8 / 24.0.
 bool rows_kernel_takes(int w_dtype, int out_dtype, int64_t rows, int64_t K, int64_t N, int flags) {
-    if (w_dtype == TTB_BFLOAT16 || out_dtype != TTB_BFLOAT16 || (flags & (TTB_MM_FORCE_GENERIC | TTB_MM_DECODE_SMEM_OPERAND))) return false;
+    // (under TTB_MM_DETERMINISTIC a call gives the bytes of the same stage of a sequence, which the decode kernel computes)
+    if (w_dtype == TTB_BFLOAT16 || out_dtype != TTB_BFLOAT16 || (flags & (TTB_MM_FORCE_GENERIC | TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_DETERMINISTIC))) return false;
     constexpr int64_t kSms = 148;
-    if (rows == 64) return (N + 127) / 128 * 2 <= kSms;
+    if (rows == 64) return (N + 127) / 128 * 2 <= kSms && K <= 8192;
     if (rows < 96) return false;
-    return !(prefill_supported(w_dtype, rows, K, N) && rows * N / 65536 * 4 >= kSms * 3);
+    if (!prefill_supported(w_dtype, rows, K, N)) return true;
+    const int64_t blocks = rows * N / 65536;
+    const bool whole_rounds = w_dtype == TTB_BFLOAT8_B && blocks >= 5 * kSms && blocks % kSms * 4 < kSms;
+    const bool one_short_round = blocks * 4 >= kSms * 3 && blocks <= kSms && K <= 2048;
+    return !(whole_rounds || one_short_round);
 }
 
 // Row ranges of one matmul and the tensor-core kernel that takes each: the decode kernels serve up to 256 rows, the prefill

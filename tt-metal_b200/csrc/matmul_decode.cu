@@ -545,7 +545,7 @@ extern "C" int32_t ttb_matmul_multi(const void *a, int32_t a_dtype, int32_t coun
     // bfloat16 results of 96 rows and more, of one rank and not gated: the kernel that expands a weight once for all its rows (us
     // before / now: 96 x 4096 x [4096, 1024, 1024] 19.5 / 18.5, 128 rows 21.5 / 18.6, 256 rows 39.9 / 24.6, 128 x 8192 x [28672,
     // 28672] 270 / 155).
-    if (rows >= 96 && out_dtype == TTB_BFLOAT16 && !gather && !wait && !(flags & (TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_GATED))) {
+    if (rows >= 96 && out_dtype == TTB_BFLOAT16 && !gather && !wait && !(flags & (TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_GATED | TTB_MM_DETERMINISTIC))) {
         int *status = nullptr;
         if (int32_t rc = status_word_address(&status)) return rc;
         return launch_matmul_rows(a, count, w, w_dtype, bias, out, out_dtype, rows, K, N, act, flags, status, (cudaStream_t)stream);

@@ -1,4 +1,4 @@
-// Matmul for middling row counts (large decode batches, short prompts; any size above that the prefill kernel does not take):
+// Matmul for middling and large row counts (large decode batches, prompts; matmul.cu has the rule):
 // out_j[rows, N_j] = act(a[rows, K] x W_j[K, N_j] + bias_j) for up to four weights W_j that share the activation, in packed bfloat8_b / bfloat4_b tiles; rows, K and N multiples of 32.
 //
 // "Swap-AB", as in the decode kernels: the MMA's M dimension (128 TMEM lanes) runs over weight columns, its N dimension over up
@@ -21,7 +21,7 @@
 // MMAs are 64, 128, 192 and 256 (kernel counters: no pipe above 40 %). Groups of one or two K blocks were slower: 690 and 610
 // clocks for 256 rows. Before, as one to three launches of the decode and prefill kernels, and now, microseconds a launch from a
 // graph: 128 x 4096 x 14336 bfloat4_b 46.2 / 28.2, 352 x 4544 x 4672 48.2 / 22.8, 512 x 4096 x 4096 74.8 / 24.0, 512 x 1024 x 1024
-// 27.0 / 9.9, 256 x 8192 x 8192 71.6 / 39.8, 64 x 4096 x 1024 15.3 / 8.8.
+// 27.0 / 9.9, 256 x 8192 x 8192 71.6 / 39.8, 64 x 4096 x 1024 15.3 / 8.8, 1536 x 4096 x 14336 220 / 176.
 // Every mbarrier wait is bounded; a wait that runs out raises a status word instead of hanging.
 #include "decode_common.cuh"
 #include "expand_tmem.cuh"
