@@ -297,3 +297,21 @@ def test_matmul_plan_names_the_kernels_without_a_gpu():
     assert plan(32, 1024, 512, cabi.BFLOAT16)[0] == 0          # bf16 weights: the shape-generic kernel
     assert plan(32, 4544, 18176, flags=cabi.MM_FORCE_GENERIC)[0] == 0
     assert lib.cdll.ttb_matmul_plan(cabi.BFLOAT8_B, 1, 32, 64, 128, 0, None, 5) == -1
+
+
+@pytest.mark.parametrize("rows", [32, 96, 256])
+@pytest.mark.parametrize("operand", ["a", "w", "out"])
+def test_misaligned_tensors_of_several_weights_are_refused_before_any_launch(rows, operand):
+    """Every tensor of ttb_matmul_multi and of a ttb_matmul_sequence stage has to start on 16 bytes: the kernels copy them in pieces of
+    that size. The addresses here are never used: the refusal comes before any CUDA call."""
+    import ctypes
+    import cabi
+    lib = cabi.load()
+    at = {"a": 1 << 16, "w": 1 << 20, "out": 1 << 24}
+    at[operand] += 2
+    w, out, N = (ctypes.c_void_p * 2)(1 << 21, at["w"]), (ctypes.c_void_p * 2)(1 << 25, at["out"]), (ctypes.c_int64 * 2)(128, 256)
+    rc = lib.cdll.ttb_matmul_multi(at["a"], cabi.BFLOAT16, 2, w, cabi.BFLOAT8_B, None, out, cabi.BFLOAT16, 1, rows, 512, N, 0, 0, None, 0, None, None, None)
+    assert rc == -1 and b"aligned" in lib.cdll.ttb_last_error()
+    st = cabi.matmul_stage(at["a"], list(w), list(out), 512, list(N))
+    rc = lib.cdll.ttb_matmul_sequence(ctypes.byref(st), 1, cabi.BFLOAT16, cabi.BFLOAT8_B, 1, rows, 0, None, 0, None)
+    assert rc == -1 and b"aligned" in lib.cdll.ttb_last_error()

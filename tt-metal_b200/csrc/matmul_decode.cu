@@ -511,6 +511,7 @@ static int32_t validate_multi(const char *who, const void *a, int32_t a_dtype, i
     if (out_dtype != TTB_BFLOAT16 && out_dtype != TTB_FLOAT32) return fail(TTB_E_UNSUPPORTED, "%s: output must be bfloat16 or float32", who);
     if (rows <= 0 || K <= 0 || rows % 32 || K % 32) return fail(TTB_E_INVALID, "%s: batch, M, K must be positive and M, K multiples of 32", who);
     if (act < TTB_ACT_NONE || act > TTB_ACT_SILU) return fail(TTB_E_INVALID, "%s: unknown activation %d", who, act);
+    if (reinterpret_cast<uintptr_t>(a) & 15) return fail(TTB_E_INVALID, "%s: tensors must be 16-byte aligned", who);
     for (int j = 0; j < count; ++j) {
         if (!w[j] || (!out[j] && !(gather && j == 0) && !((flags & TTB_MM_GATED) && j == 1)))
             return fail(TTB_E_INVALID, "%s: null tensor pointer for weight %d", who, j);
