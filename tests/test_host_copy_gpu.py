@@ -29,6 +29,31 @@ def test_round_trip(ttb, bytes_, skip):
     round_trip(ttb, bytes_, skip, pinned=True)
 
 
+@pytest.mark.parametrize("stream", [None, 2, "own"])
+def test_copies_are_ordered_after_the_streams_work(ttb, stream):
+    """A kernel's worth of copies writes what is read back, and reads what is overwritten, on the default stream, the per-thread
+    default stream (handle 2) and one of the caller's."""
+    import torch
+    n, own = 24 * MB, torch.cuda.Stream()
+    s = own.cuda_stream if stream == "own" else stream
+    big = torch.zeros(2, 512 * MB, dtype=torch.uint8, device="cuda")
+    dev, old = torch.zeros(n, dtype=torch.uint8, device="cuda"), torch.empty(n, dtype=torch.uint8, device="cuda")
+    src, dst = torch.full((n,), 3, dtype=torch.uint8), torch.zeros(n, dtype=torch.uint8)
+    torch.cuda.synchronize()
+    for _ in range(20):                                        # about 4 ms ahead of what the copy has to wait for
+        ttb.check(ttb.cdll.ttb_memcpy_d2d(big[0].data_ptr(), big[1].data_ptr(), 512 * MB, s))
+    ttb.check(ttb.cdll.ttb_memset(dev.data_ptr(), 7, n, s))
+    ttb.check(ttb.cdll.ttb_memcpy_d2h(dst.data_ptr(), dev.data_ptr(), n, s))
+    ttb.check(ttb.cdll.ttb_stream_synchronize(s))
+    assert bool((dst == 7).all())
+    for _ in range(20):
+        ttb.check(ttb.cdll.ttb_memcpy_d2d(big[0].data_ptr(), big[1].data_ptr(), 512 * MB, s))
+    ttb.check(ttb.cdll.ttb_memcpy_d2d(old.data_ptr(), dev.data_ptr(), n, s))
+    ttb.check(ttb.cdll.ttb_memcpy_h2d(dev.data_ptr(), src.data_ptr(), n, s))
+    ttb.check(ttb.cdll.ttb_stream_synchronize(s))
+    assert bool((old == 7).all()) and bool((dev == 3).all())
+
+
 def test_several_threads(ttb):
     failures = []
 

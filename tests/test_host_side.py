@@ -1,0 +1,53 @@
+"""The library's host code on a fake CUDA runtime (fake_cudart.cpp): its own objects, linked against functions that copy with
+memcpy and write launches down. What goes wrong with threads, streams, contexts and captures shows here without a GPU."""
+import ctypes
+import glob
+import os
+import subprocess
+import sys
+import threading
+
+import pytest
+
+import cabi
+
+MB = 1 << 20
+PER_THREAD_STREAM = 2        # cudaStreamPerThread
+
+
+def build_fake(directory):
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("ttb_build", os.path.join(cabi.ROOT, "tt-metal_b200", "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    build.build_libttb()
+    so = os.path.join(directory, "libttb_fake.so")
+    # (-Bsymbolic: its own copies of the runtime, whatever else the process has loaded)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-Wno-attributes", "-I/usr/local/cuda/include",
+                    os.path.join(cabi.ROOT, "tests", "fake_cudart.cpp")] + sorted(glob.glob(os.path.join(build.OBJ, "*.o"))) +
+                   ["-o", so, "-lpthread", "-ldl"], check=True)
+    return so
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    lib = cabi.Lib(build_fake(str(tmp_path_factory.mktemp("fake"))))
+    lib.cdll.fake_log.restype = ctypes.c_char_p
+    return lib
+
+
+def round_trip(lib, nbytes, stream=None):
+    """Host to device and back; both host buffers are pageable, the device's is plain memory here."""
+    src, dev, dst = os.urandom(nbytes), ctypes.create_string_buffer(nbytes), ctypes.create_string_buffer(nbytes)
+    lib.check(lib.cdll.ttb_memcpy_h2d(dev, src, nbytes, stream))
+    lib.check(lib.cdll.ttb_memcpy_d2h(dst, dev, nbytes, stream))
+    assert dst.raw == src
+
+
+def test_copies_on_the_per_thread_stream_stay_on_the_callers_thread(fake):
+    """The handle names another stream on every thread: whoever enqueues on it elsewhere is not ordered after the caller's work."""
+    fake.cdll.fake_stream_users()
+    round_trip(fake, 9 * MB + 5, PER_THREAD_STREAM)
+    assert fake.cdll.fake_stream_users() == 1
+    round_trip(fake, 9 * MB + 5)
+    assert fake.cdll.fake_stream_users() > 1      # the legacy stream is the same on all of them

@@ -76,9 +76,10 @@ cudaError_t copy_chunks(int t, int threads, int device, uint8_t *dev, uint8_t *h
 }  // namespace
 
 // Copies through the pinned buffers if that is the better way, complete on return; false: the caller copies as usual. What
-// belongs to a capture, small or already pinned is left alone, and so is a copy that meets another one at work.
+// belongs to a capture, small or already pinned is left alone, and so is a copy that meets another one at work. The handle of
+// the per-thread default stream names another stream on each of the threads here, none of them ordered after the caller's work.
 bool copy_staged(void *dev, void *host, size_t bytes, bool to_device, cudaStream_t stream, cudaError_t &error) {
-    if (bytes < kMinBytes || !pageable(host)) return false;
+    if (bytes < kMinBytes || stream == cudaStreamPerThread || !pageable(host)) return false;
     cudaStreamCaptureStatus capturing;
     if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
         (void)cudaGetLastError();
