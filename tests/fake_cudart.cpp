@@ -36,10 +36,9 @@ cudaError_t unsafe() {   // a call that another thread's capture in global mode 
     }
     return cudaSuccess;
 }
-cudaError_t used(cudaStream_t s) {   // stream 0x300 belongs to the other context
+void used(cudaStream_t s) {
     std::lock_guard<std::mutex> l(g_mutex);
     g_users.insert({pthread_self(), s});
-    return s == (cudaStream_t)0x300 && current() != g_other ? cudaErrorInvalidResourceHandle : cudaSuccess;
 }
 CUresult ctx_get_current(CUcontext *c) { *c = t_context; return CUDA_SUCCESS; }
 CUresult ctx_set_current(CUcontext c) { t_context = c; return CUDA_SUCCESS; }
@@ -134,7 +133,7 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t st) {
-    if (cudaError_t e = used(st)) return e;
+    used(st);
     memcpy(d, s, n);
     return cudaSuccess;
 }
@@ -143,7 +142,10 @@ cudaError_t cudaMemcpyFromSymbol(void *, const void *, size_t, size_t, cudaMemcp
 cudaError_t cudaMemcpyToSymbol(const void *, const void *, size_t, size_t, cudaMemcpyKind) { return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { *e = (cudaEvent_t)0x1; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t s) { return used(s); }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t s) {   // stream 0x300 belongs to the other context, every event to the current one
+    used(s);
+    return s == (cudaStream_t)0x300 && current() != g_other ? cudaErrorInvalidResourceHandle : cudaSuccess;
+}
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return unsafe(); }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return unsafe(); }
 cudaError_t cudaIpcGetMemHandle(cudaIpcMemHandle_t *, void *) { return cudaErrorNotSupported; }

@@ -51,3 +51,26 @@ def test_copies_on_the_per_thread_stream_stay_on_the_callers_thread(fake):
     assert fake.cdll.fake_stream_users() == 1
     round_trip(fake, 9 * MB + 5)
     assert fake.cdll.fake_stream_users() > 1      # the legacy stream is the same on all of them
+
+
+def test_a_stream_of_another_context_takes_the_plain_copy(fake):
+    """Handle 0x300 belongs to a context that is not current (another device's, for instance): events of the current one cannot be
+    recorded there."""
+    fake.cdll.fake_stream_users()
+    round_trip(fake, 8 * MB, 0x300)
+    assert fake.cdll.fake_stream_users() == 1
+
+
+def test_a_callers_own_context_stays_current_and_is_the_helpers(fake):
+    """A context made through the driver API, not the device's primary one: the helper threads work in it, and it stays current."""
+    def work():
+        fake.cdll.fake_context(1)
+        before = fake.cdll.fake_set_device_calls()
+        round_trip(fake, 8 * MB + 1, 0x300)                                  # a stream of that context
+        result.extend([fake.cdll.fake_context_is_other(), fake.cdll.fake_set_device_calls() - before])
+
+    result = []
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert result == [1, 0]

@@ -10,7 +10,8 @@
 #include <mutex>
 #include <system_error>
 #include <thread>
-#include <vector>
+
+#include <cuda.h>
 
 #include "common.cuh"
 
@@ -40,12 +41,33 @@ bool pageable(const void *p) {
     return a.type == cudaMemoryTypeUnregistered;
 }
 
+// The driver's view of contexts, through the runtime's entry points (no link against the driver library).
+struct Contexts {
+    CUresult (*get_current)(CUcontext *) = nullptr;
+    CUresult (*set_current)(CUcontext) = nullptr;
+    CUresult (*of_stream)(CUstream, CUcontext *) = nullptr;
+    bool ok = false;
+    Contexts() {
+        auto find = [](const char *name, void **fn) {
+            cudaDriverEntryPointQueryResult r;
+            return cudaGetDriverEntryPoint(name, fn, cudaEnableDefault, &r) == cudaSuccess && r == cudaDriverEntryPointSuccess && *fn;
+        };
+        ok = find("cuCtxGetCurrent", reinterpret_cast<void **>(&get_current)) && find("cuCtxSetCurrent", reinterpret_cast<void **>(&set_current)) &&
+             find("cuStreamGetCtx", reinterpret_cast<void **>(&of_stream));
+        if (!ok) (void)cudaGetLastError();
+    }
+};
+const Contexts &contexts() {
+    static const Contexts c;
+    return c;
+}
+
 // Chunks t, t + threads, ... of the copy, alternating between this thread's two pinned buffers.
-cudaError_t copy_chunks(int t, int threads, int device, uint8_t *dev, uint8_t *host, size_t bytes, bool to_device, uint8_t *pinned, cudaStream_t stream) {
+cudaError_t copy_chunks(int t, int threads, uint8_t *dev, uint8_t *host, size_t bytes, bool to_device, uint8_t *pinned, cudaStream_t stream) {
     cudaEvent_t done[kSlots] = {};
     uint8_t *target[kSlots] = {};    // towards the host: where the chunk in flight in a buffer belongs, and its size
     size_t size[kSlots] = {};
-    cudaError_t e = cudaSetDevice(device);
+    cudaError_t e = cudaSuccess;
     for (int s = 0; s < kSlots && e == cudaSuccess; ++s) e = cudaEventCreateWithFlags(&done[s], cudaEventDisableTiming);
     auto drain = [&](int s) {        // the buffer's previous chunk has been moved on
         if (e == cudaSuccess && size[s]) {
@@ -78,6 +100,8 @@ cudaError_t copy_chunks(int t, int threads, int device, uint8_t *dev, uint8_t *h
 // Copies through the pinned buffers if that is the better way, complete on return; false: the caller copies as usual. What
 // belongs to a capture, small or already pinned is left alone, and so is a copy that meets another one at work. The handle of
 // the per-thread default stream names another stream on each of the threads here, none of them ordered after the caller's work.
+// The helper threads work in the caller's context (which need not be its device's primary one); a stream of another context, whose
+// work the events here could not mark, is left alone too.
 bool copy_staged(void *dev, void *host, size_t bytes, bool to_device, cudaStream_t stream, cudaError_t &error) {
     if (bytes < kMinBytes || stream == cudaStreamPerThread || !pageable(host)) return false;
     cudaStreamCaptureStatus capturing;
@@ -85,8 +109,10 @@ bool copy_staged(void *dev, void *host, size_t bytes, bool to_device, cudaStream
         (void)cudaGetLastError();
         return false;
     }
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    CUcontext context = nullptr, owner = nullptr;
+    if (!contexts().ok || contexts().get_current(&context) != CUDA_SUCCESS || !context || contexts().of_stream(stream, &owner) != CUDA_SUCCESS ||
+        owner != context)
+        return false;
     std::unique_lock<std::mutex> lock(g_staging.mutex, std::try_to_lock);
     if (!lock.owns_lock()) return false;
     if (!g_staging.base) {
@@ -100,12 +126,18 @@ bool copy_staged(void *dev, void *host, size_t bytes, bool to_device, cudaStream
     const int threads = (int)std::min<size_t>({(size_t)kThreads, bytes / (2 * kChunk), std::max<size_t>(1, std::thread::hardware_concurrency())});
     cudaError_t results[kThreads] = {};
     auto work = [&](int t) {
-        results[t] = copy_chunks(t, threads, device, (uint8_t *)dev, (uint8_t *)host, bytes, to_device, g_staging.base + t * kSlots * kChunk, stream);
+        results[t] = copy_chunks(t, threads, (uint8_t *)dev, (uint8_t *)host, bytes, to_device, g_staging.base + t * kSlots * kChunk, stream);
     };
     std::thread pool[kThreads];
     int started = 1;
     try {
-        for (; started < threads; ++started) pool[started] = std::thread(work, started);
+        for (; started < threads; ++started)
+            pool[started] = std::thread([&, t = started] {
+                if (contexts().set_current(context) == CUDA_SUCCESS)
+                    work(t);
+                else
+                    results[t] = cudaErrorInvalidValue;
+            });
     } catch (const std::system_error &) {   // no more threads: this one takes their chunks as well
     }
     work(0);
