@@ -74,3 +74,16 @@ def test_a_callers_own_context_stays_current_and_is_the_helpers(fake):
     t.start()
     t.join()
     assert result == [1, 0]
+
+
+def test_a_first_large_copy_leaves_another_threads_capture_intact(fake):
+    """While some thread captures in global mode, allocations and waits of the others are forbidden calls that end its capture,
+    unless they declare themselves relaxed. The plain copy made none; its pinned buffers, allocated by the first copy, may not either."""
+    fake.cdll.fake_reset_device()
+    fake.cdll.fake_capture(1)
+    try:
+        round_trip(fake, 8 * MB)
+        assert fake.cdll.fake_violations() == 0
+        assert fake.cdll.ttb_stream_synchronize(None) != 0 and fake.cdll.fake_violations() == 1   # the caller's own mode is as it was
+    finally:
+        fake.cdll.fake_capture(0)

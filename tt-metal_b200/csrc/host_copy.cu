@@ -62,11 +62,20 @@ const Contexts &contexts() {
     return c;
 }
 
+// While some thread captures in global mode, the others' allocations and waits are forbidden unless they declare themselves
+// relaxed, and end that thread's capture. Nothing here belongs to a capture.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Chunks t, t + threads, ... of the copy, alternating between this thread's two pinned buffers.
 cudaError_t copy_chunks(int t, int threads, uint8_t *dev, uint8_t *host, size_t bytes, bool to_device, uint8_t *pinned, cudaStream_t stream) {
     cudaEvent_t done[kSlots] = {};
     uint8_t *target[kSlots] = {};    // towards the host: where the chunk in flight in a buffer belongs, and its size
     size_t size[kSlots] = {};
+    const RelaxedCapture relaxed;
     cudaError_t e = cudaSuccess;
     for (int s = 0; s < kSlots && e == cudaSuccess; ++s) e = cudaEventCreateWithFlags(&done[s], cudaEventDisableTiming);
     auto drain = [&](int s) {        // the buffer's previous chunk has been moved on
@@ -115,6 +124,7 @@ bool copy_staged(void *dev, void *host, size_t bytes, bool to_device, cudaStream
         return false;
     std::unique_lock<std::mutex> lock(g_staging.mutex, std::try_to_lock);
     if (!lock.owns_lock()) return false;
+    const RelaxedCapture relaxed;
     if (!g_staging.base) {
         void *p = nullptr;
         if (cudaHostAlloc(&p, kChunk * kThreads * kSlots, cudaHostAllocPortable) != cudaSuccess) {
