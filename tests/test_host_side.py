@@ -87,3 +87,12 @@ def test_a_first_large_copy_leaves_another_threads_capture_intact(fake):
         assert fake.cdll.ttb_stream_synchronize(None) != 0 and fake.cdll.fake_violations() == 1   # the caller's own mode is as it was
     finally:
         fake.cdll.fake_capture(0)
+
+
+def test_pinned_buffers_are_allocated_again_once_their_context_is_gone(fake):
+    """cudaDeviceReset and a destroyed context take the pinned buffers with them."""
+    round_trip(fake, 8 * MB)
+    assert fake.cdll.fake_pinned() == 1
+    fake.cdll.fake_reset_device()
+    round_trip(fake, 8 * MB)
+    assert fake.cdll.fake_pinned() == 1

@@ -32,13 +32,13 @@ struct Staging {
 };
 Staging g_staging;
 
-bool pageable(const void *p) {
+bool memory_is(const void *p, cudaMemoryType type) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
-    return a.type == cudaMemoryTypeUnregistered;
+    return a.type == type;
 }
 
 // The driver's view of contexts, through the runtime's entry points (no link against the driver library).
@@ -112,7 +112,7 @@ cudaError_t copy_chunks(int t, int threads, uint8_t *dev, uint8_t *host, size_t 
 // The helper threads work in the caller's context (which need not be its device's primary one); a stream of another context, whose
 // work the events here could not mark, is left alone too.
 bool copy_staged(void *dev, void *host, size_t bytes, bool to_device, cudaStream_t stream, cudaError_t &error) {
-    if (bytes < kMinBytes || stream == cudaStreamPerThread || !pageable(host)) return false;
+    if (bytes < kMinBytes || stream == cudaStreamPerThread || !memory_is(host, cudaMemoryTypeUnregistered)) return false;
     cudaStreamCaptureStatus capturing;
     if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
         (void)cudaGetLastError();
@@ -125,6 +125,7 @@ bool copy_staged(void *dev, void *host, size_t bytes, bool to_device, cudaStream
     std::unique_lock<std::mutex> lock(g_staging.mutex, std::try_to_lock);
     if (!lock.owns_lock()) return false;
     const RelaxedCapture relaxed;
+    if (g_staging.base && !memory_is(g_staging.base, cudaMemoryTypeHost)) g_staging.base = nullptr;   // went with its context (cudaDeviceReset)
     if (!g_staging.base) {
         void *p = nullptr;
         if (cudaHostAlloc(&p, kChunk * kThreads * kSlots, cudaHostAllocPortable) != cudaSuccess) {
