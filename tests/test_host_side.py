@@ -96,3 +96,16 @@ def test_pinned_buffers_are_allocated_again_once_their_context_is_gone(fake):
     fake.cdll.fake_reset_device()
     round_trip(fake, 8 * MB)
     assert fake.cdll.fake_pinned() == 1
+
+
+@pytest.mark.parametrize("failing", range(4))
+def test_a_thread_that_cannot_be_made_is_done_without(fake, failing):
+    """std::thread's own allocation fails (std::bad_alloc, not std::system_error): no exception leaves the C entry point, the threads
+    that did start are joined, and the bytes are right."""
+    src, dev = os.urandom(16 * MB + 3), ctypes.create_string_buffer(16 * MB + 3)
+    fake.cdll.fake_fail_new(failing)
+    try:
+        rc = fake.cdll.ttb_memcpy_h2d(dev, src, len(src), None)
+    finally:
+        fake.cdll.fake_fail_new(-1)
+    assert rc == 0 and dev.raw == src

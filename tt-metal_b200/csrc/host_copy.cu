@@ -8,7 +8,6 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 #include <cuda.h>
@@ -149,7 +148,7 @@ bool copy_staged(void *dev, void *host, size_t bytes, bool to_device, cudaStream
                 else
                     results[t] = cudaErrorInvalidValue;
             });
-    } catch (const std::system_error &) {   // no more threads: this one takes their chunks as well
+    } catch (...) {   // no more threads, or no memory for one: this one takes their chunks as well
     }
     work(0);
     for (int t = started; t < threads; ++t) work(t);
