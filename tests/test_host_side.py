@@ -109,3 +109,28 @@ def test_a_thread_that_cannot_be_made_is_done_without(fake, failing):
     finally:
         fake.cdll.fake_fail_new(-1)
     assert rc == 0 and dev.raw == src
+
+
+@pytest.mark.parametrize("w_dtype", [cabi.BFLOAT16, cabi.BFLOAT8_B, cabi.BFLOAT4_B])
+def test_first_calls_of_several_threads_set_a_kernel_up_once(tmp_path, w_dtype):
+    """The launch reads what the set-up of its device counted: a second thread waits until that is there. (A process of its own: the
+    set-up is done once.)"""
+    code = """if True:
+        import ctypes, sys, threading
+        sys.path.insert(0, %r)
+        import cabi
+        lib = cabi.Lib(%r)
+        lib.cdll.fake_log.restype = ctypes.c_char_p
+        lib.cdll.fake_slow_us(20000)
+        go, codes = threading.Barrier(4), []
+        def work():
+            go.wait()
+            codes.append(lib.cdll.ttb_matmul(4096, 0, 8192, %d, None, 16384, 0, 1, 128, 4096, 256, 0, 8, None, 0, None))
+        threads = [threading.Thread(target=work) for _ in range(4)]
+        [t.start() for t in threads]; [t.join() for t in threads]
+        log = lib.cdll.fake_log().decode().split()
+        assert codes == [0] * 4 and len(log) == 4 and len(set(log)) == 1, (codes, log)
+        print(lib.cdll.fake_most_configured())
+    """ % (os.path.join(cabi.ROOT, "tests"), build_fake(str(tmp_path)), w_dtype)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "1", r.stdout + r.stderr

@@ -2,9 +2,11 @@
 // block-float code <-> fp32-bit conversions used by the conversion and matmul kernels.
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 
 #include "ttb.h"
 
@@ -28,6 +30,23 @@ int32_t fail(int32_t code, const char *fmt, ...);
         if (e__ != cudaSuccess)                                                              \
             return ::ttb::fail(TTB_E_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e__)); \
     } while (0)
+
+// Set-up that the first call does and the others wait for (all of them again after one that failed).
+class Once {
+    std::mutex mutex_;
+    std::atomic<bool> done_{false};
+
+   public:
+    template <typename F>
+    int32_t run(F set_up) {
+        if (done_.load(std::memory_order_acquire)) return TTB_OK;
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (done_.load(std::memory_order_relaxed)) return TTB_OK;
+        if (int32_t rc = set_up()) return rc;
+        done_.store(true, std::memory_order_release);
+        return TTB_OK;
+    }
+};
 
 constexpr int kTile = 32;
 constexpr int kTileElems = 1024;

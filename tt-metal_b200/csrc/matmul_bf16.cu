@@ -375,38 +375,39 @@ int32_t launch_matmul_bf16(const void *a, const void *w, const void *bias, void 
     p.mt = (int)mt; p.nt = (int)nt; p.tiles = (int)tiles;
     p.nstages = (int)((K + BK - 1) / BK);
     p.chunk = out_dtype == TTB_FLOAT32 ? 1 : 4;
-    int dev = 0, sms = 148;
+    int dev = 0;
     TTB_CUDA_TRY(cudaGetDevice(&dev));
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     static struct {
-        bool configured;
-        int clusters[9];   // clusters of 2, 4 and 8 blocks that run at the same time
-    } devices[64] = {};
+        Once once;
+        int sms, clusters[9];   // multiprocessors; clusters of 2, 4 and 8 blocks that run at the same time
+    } devices[64];
     if (dev < 0 || dev >= 64) return fail(TTB_E_UNSUPPORTED, "ttb_matmul: device index %d is out of range", dev);
     auto &d = devices[dev];
-    if (!d.configured) {
-        TTB_CUDA_TRY(cudaFuncSetAttribute(matmul_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        for (int c = 2; c <= 8; c *= 2) {
-            cudaLaunchConfig_t q = {};
-            q.gridDim = dim3((unsigned)(sms / c * c));
-            q.blockDim = dim3(kThreads);
-            q.dynamicSmemBytes = kSmemBytes;
-            cudaLaunchAttribute ca[1];
-            ca[0].id = cudaLaunchAttributeClusterDimension;
-            ca[0].val.clusterDim.x = (unsigned)c;
-            ca[0].val.clusterDim.y = ca[0].val.clusterDim.z = 1;
-            q.attrs = ca;
-            q.numAttrs = 1;
-            TTB_CUDA_TRY(cudaOccupancyMaxActiveClusters(&d.clusters[c], matmul_bf16_kernel, &q));
-        }
-        d.configured = true;
-    }
+    if (int32_t rc = d.once.run([&]() -> int32_t {
+            TTB_CUDA_TRY(cudaFuncSetAttribute(matmul_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+            TTB_CUDA_TRY(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
+            for (int c = 2; c <= 8; c *= 2) {
+                cudaLaunchConfig_t q = {};
+                q.gridDim = dim3((unsigned)(d.sms / c * c));
+                q.blockDim = dim3(kThreads);
+                q.dynamicSmemBytes = kSmemBytes;
+                cudaLaunchAttribute ca[1];
+                ca[0].id = cudaLaunchAttributeClusterDimension;
+                ca[0].val.clusterDim.x = (unsigned)c;
+                ca[0].val.clusterDim.y = ca[0].val.clusterDim.z = 1;
+                q.attrs = ca;
+                q.numAttrs = 1;
+                TTB_CUDA_TRY(cudaOccupancyMaxActiveClusters(&d.clusters[c], matmul_bf16_kernel, &q));
+            }
+            return TTB_OK;
+        }))
+        return rc;
     // Clusters share a tile while all of them run at the same time and each block keeps at least four stages (the exchange of
     // partial sums costs about as much as two).
     p.split = 1;
     while (p.split < 8 && tiles <= d.clusters[p.split * 2] && p.nstages / (p.split * 2) >= 4) p.split *= 2;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(p.split > 1 ? tiles * p.split : tiles < sms ? tiles : sms));
+    cfg.gridDim = dim3((unsigned)(p.split > 1 ? tiles * p.split : tiles < d.sms ? tiles : d.sms));
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = stream;

@@ -397,14 +397,12 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
 }
 
 struct Device {
-    bool configured[2][2];   // per weight format and chunk size
+    Once once;
     int sms, clusters[9];    // multiprocessors; clusters of 2..8 blocks that run at the same time
 };
 
 template <int FMT, int BR>
 int32_t configure(Device &d, int dev) {
-    bool &done = d.configured[FMT == TTB_BFLOAT4_B][BR == 256];
-    if (done) return TTB_OK;
     constexpr int smem = Layout<FMT, BR>::total;
     TTB_CUDA_TRY(cudaFuncSetAttribute(matmul_rows_kernel<FMT, BR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int sms = 0;
@@ -425,7 +423,6 @@ int32_t configure(Device &d, int dev) {
         d.clusters[c] = n;
     }
     d.sms = sms;
-    done = true;
     return TTB_OK;
 }
 
@@ -468,13 +465,16 @@ int32_t launch_all(Args &p, int tiles, int split, int sms, bool overlap, cudaStr
 
 template <int FMT>
 int32_t launch_fmt(Args &p, bool overlap, cudaStream_t stream) {
-    static Device devices[64] = {};
+    static Device devices[64];
     int dev = 0;
     TTB_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return fail(TTB_E_UNSUPPORTED, "ttb_matmul: device index %d is out of range", dev);
     Device &d = devices[dev];
-    if (int32_t rc = configure<FMT, 192>(d, dev)) return rc;
-    if (int32_t rc = configure<FMT, 256>(d, dev)) return rc;
+    if (int32_t rc = d.once.run([&] {
+            const int32_t c = configure<FMT, 192>(d, dev);
+            return c ? c : configure<FMT, 256>(d, dev);
+        }))
+        return rc;
     // Blocks that share a tile: as many as run at the same time, each with at least eight K blocks (the exchange of the partial
     // sums costs about that much).
     auto split_for = [&](int n) {
