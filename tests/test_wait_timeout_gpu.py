@@ -97,3 +97,35 @@ def test_host_layer_raises_on_a_timeout_and_clears_its_scratch(ttb, short_waits)
     got = ttnn.to_torch(ttnn.linear(tx, tw)).float()
     # (sums over K may be added in another order from launch to launch: equal to the last bf16 digit, not to the bit)
     assert torch.allclose(got, want, rtol=2 ** -6, atol=1e-3 * float(want.abs().max()))
+
+
+@pytest.mark.parametrize("w_dtype", [cabi.BFLOAT16, cabi.BFLOAT8_B, cabi.BFLOAT4_B])
+def test_a_kernel_behind_one_that_waits_for_peers_does_not_run_out_itself(ttb, orc, w_dtype):
+    """A decode matmul waits 1.3 s for peers that never deliver, on few multiprocessors; the overlapped matmul behind it starts at
+    once on the others. Its own barriers, limited to about a second, are not to count that time: the status names the first kernel's
+    wait, and the second one's result is right."""
+    import torch
+    M, K, N = 128, 1024, 256
+    x, w_dev, w_ref = make_case(ttb, orc, 17, M, K, N, w_dtype)
+    x2, w2, _ = make_case(ttb, orc, 18, 32, 256, 128, cabi.BFLOAT8_B)
+    a, a2 = ttb.tilize(x.cuda(), 1, M, K), ttb.tilize(x2.cuda(), 1, 32, 256)
+    ws = torch.zeros(65536 + (48 << 20), dtype=torch.uint8, device="cuda")
+    out, out2 = torch.zeros(M * N, dtype=torch.bfloat16, device="cuda"), torch.zeros(32 * 128, dtype=torch.bfloat16, device="cuda")
+    run = lambda: ttb.check(ttb.cdll.ttb_matmul(a.data_ptr(), cabi.BFLOAT16, w_dev.data_ptr(), w_dtype, None, out.data_ptr(), cabi.BFLOAT16, 1, M, K, N, 0,   # noqa: E731
+                                                cabi.MM_WORKSPACE_ZEROED | cabi.MM_WEIGHTS_RESIDENT, ws.data_ptr(), ws.numel(), None))
+    run()                                                       # (set-up and module loading are over)
+    assert ttb.check_status(None) == 0
+    out.zero_()
+    counters, wt = _dead_gather_point()
+    ttb.check(ttb.set_wait_limit_cycles(2_600_000_000))
+    try:
+        ttb.check(ttb.cdll.ttb_matmul_peer(a2.data_ptr(), cabi.BFLOAT16, w2.data_ptr(), cabi.BFLOAT8_B, None, out2.data_ptr(), cabi.BFLOAT16, 1, 32, 256, 128, 0,
+                                           cabi.MM_WORKSPACE_ZEROED, ws.data_ptr(), ws.numel(), None, ctypes.byref(wt), None))
+    finally:
+        ttb.check(ttb.set_wait_limit_cycles(0))
+    run()
+    assert ttb.check_status(None) == TTB_E_TIMEOUT
+    site = int(ttb.cdll.ttb_last_error().decode().split("wait site ")[1].rstrip(")"))
+    assert site < 40, site                                      # 41.. are the second kernel's barriers
+    assert ttb.check_status(None) == 0
+    check(ttb.untilize(out, 1, M, N).reshape(M, N), x.float() @ w_ref)

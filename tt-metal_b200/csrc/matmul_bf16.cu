@@ -162,8 +162,9 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_bf16_kernel(const __grid_c
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    // The launch overlaps the previous kernel's tail (programmatic dependency); nothing above touches global memory, and the
-    // roles that do wait for that kernel first.
+    // The launch overlaps the previous kernel's tail (programmatic dependency); nothing above touches global memory, and every
+    // role waits for that kernel first: the roles that do touch it, and the issuer because its bounded waits are not to count
+    // the time of a kernel that waits for other GPUs.
     grid_dep_launch();
 
     // this block's share of a tile's K range, in stages (the same for every tile); a split gives every block at least one
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_bf16_kernel(const __grid_c
         cp_async_wait_all();   // (also after a wait that ran out: nothing is left in flight)
     } else if (warp == kMmaWarp) {
         // ---------------- MMA issuer (warp-uniform, one elected lane issues) ----------------
+        grid_dep_wait();
         const bool leader = elect_one();
         constexpr uint32_t idesc = instr_desc_bf16_f32(BM, BN, /*a_mn_major=*/false, /*b_mn_major=*/true);
         const uint64_t a_desc0 = smem_desc_sw32(sbase, kSBO), b_desc0 = smem_desc_sw32_mn(sbase + kOperandBytes, kBGroup, kSBO);

@@ -22,7 +22,8 @@
 // clocks for 256 rows. Before, as one to three launches of the decode and prefill kernels, and now, microseconds a launch from a
 // graph: 128 x 4096 x 14336 bfloat4_b 46.2 / 28.2, 352 x 4544 x 4672 48.2 / 22.8, 512 x 4096 x 4096 74.8 / 24.0, 512 x 1024 x 1024
 // 27.0 / 9.9, 256 x 8192 x 8192 71.6 / 39.8, 64 x 4096 x 1024 15.3 / 8.8, 1536 x 4096 x 14336 220 / 176.
-// Every mbarrier wait is bounded; a wait that runs out raises a status word instead of hanging.
+// Every mbarrier wait is bounded; a wait that runs out raises a status word instead of hanging. No such wait begins while it
+// depends on the previous kernel (which may itself wait for other GPUs for seconds): the role waits for that kernel first.
 #include "decode_common.cuh"
 #include "expand_tmem.cuh"
 
@@ -198,11 +199,12 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
         const int sh0 = 2 * (lane & 3);
         const uint32_t pk_quad = sbase + L::pk + quad * L::kTile;
         const uint32_t a_quad = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)kACol0;
-        int gs = 0, ps = 0;
+        int gs = 0, ps = 0, ahead = kRing;   // groups that go before the first MMA
         uint32_t ph = 0, pph = 0;
         bool ok = true;
         for (int t = first; ok && t < p.tiles; t += step) {
             for (int kb = kb0; kb < kb1; kb += kGroup) {
+                if (ahead-- == 0) grid_dep_wait();   // the MMAs wait for the previous kernel: its time is not this barrier's
                 if (!__all_sync(0xffffffffu, mbar_wait(full_p(ps), pph, abort_flag, p.status, 51) && mbar_wait(empty(gs), ph ^ 1u, abort_flag, p.status, 52))) {
                     ok = false;
                     break;
@@ -228,13 +230,14 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
     } else if (warp == kProducerWarp) {
         // ---------------- packed weight tiles -> shared memory ----------------
         const bool leader = elect_one();
-        int s = 0;
+        int s = 0, ahead = kPRing + kRing;
         uint32_t ph = 0;
         bool ok = true;
         for (int t = first; ok && t < p.tiles; t += step) {
             int w;
             const int nt = column_tile_of(t, w);
             for (int kb = kb0; kb < kb1; kb += kGroup) {
+                if (ahead-- == 0) grid_dep_wait();   // (as above: the expand warps have emptied kRing groups by then)
                 if (!__all_sync(0xffffffffu, mbar_wait(empty_p(s), ph ^ 1u, abort_flag, p.status, 53))) { ok = false; break; }
                 if (leader) {
                     // (always a whole box: what lies beyond the weight reads as zeros, a surplus K block is not expanded)
@@ -286,6 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
         cp_async_wait_all();   // nothing of this warp's is in flight at the teardown
     } else if (warp == kMmaWarp) {
         // ---------------- MMA issuer: A (weights) from tensor memory, B (activations) from shared memory ----------------
+        grid_dep_wait();   // (the activations come after it: no bounded wait is to count the previous kernel's time)
         const bool leader = elect_one();
         const uint64_t x_desc0 = smem_desc_sw32(sbase + L::x, kX_SBO);
         const uint32_t x_lo0 = (uint32_t)x_desc0, x_hi = (uint32_t)(x_desc0 >> 32);
