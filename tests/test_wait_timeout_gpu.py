@@ -129,3 +129,22 @@ def test_a_kernel_behind_one_that_waits_for_peers_does_not_run_out_itself(ttb, o
     assert site < 40, site                                      # 41.. are the second kernel's barriers
     assert ttb.check_status(None) == 0
     check(ttb.untilize(out, 1, M, N).reshape(M, N), x.float() @ w_ref)
+
+
+def test_the_middling_rows_kernel_takes_the_limit(ttb):
+    """One tile whose K range keeps its blocks busy for about a millisecond: the epilogue's wait for it runs out under the shortest limit
+    (half a millisecond) and not under the default one. (An operand of zeros: only the time counts.)"""
+    import torch
+    M, K, N = 320, 1 << 21, 128
+    a, w = torch.zeros(M * K, dtype=torch.bfloat16, device="cuda"), torch.zeros(K * N // 1024 * 1088, dtype=torch.uint8, device="cuda")
+    out = torch.full((M * N,), 7.0, dtype=torch.bfloat16, device="cuda")
+    run = lambda: ttb.check(ttb.cdll.ttb_matmul(a.data_ptr(), cabi.BFLOAT16, w.data_ptr(), cabi.BFLOAT8_B, None, out.data_ptr(), cabi.BFLOAT16, 1, M, K, N, 0, 0,   # noqa: E731
+                                                None, 0, None))
+    ttb.check(ttb.set_wait_limit_cycles(1))
+    try:
+        run()
+    finally:
+        ttb.check(ttb.set_wait_limit_cycles(0))
+    assert ttb.check_status(None) == TTB_E_TIMEOUT and b"wait site 57" in ttb.cdll.ttb_last_error()
+    run()
+    assert ttb.check_status(None) == 0 and not bool(out.any())

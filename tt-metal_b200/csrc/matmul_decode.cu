@@ -12,6 +12,8 @@ __device__ int g_status_word = 0;
 // Limit of the bounded device-side waits in SM clocks; 0 = each wait's built-in default. Read at launch time.
 static long long g_wait_limit_cycles = 0;
 long long wait_limit_cycles() { return g_wait_limit_cycles; }
+// ... of the pipeline barriers of a kernel that waits for no peers itself.
+long long barrier_limit_cycles() { return g_wait_limit_cycles > 0 ? 2 * g_wait_limit_cycles + 1000000LL : 2000000000LL; }
 
 using namespace decode_smem;
 

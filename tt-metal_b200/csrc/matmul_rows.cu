@@ -28,6 +28,7 @@
 #include "expand_tmem.cuh"
 
 namespace ttb {
+long long barrier_limit_cycles();
 namespace {
 
 using namespace ptx;
@@ -80,6 +81,7 @@ struct alignas(64) Args {
     int split;              // blocks (= cluster size) that share a tile's K range
     int act, out_dtype, a_row_major, out_row_major;
     int *status;
+    long long wait_limit;   // of every barrier wait, in SM clocks
 };
 
 __device__ __forceinline__ void cluster_sync() {
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
         for (int t = first; ok && t < p.tiles; t += step) {
             for (int kb = kb0; kb < kb1; kb += kGroup) {
                 if (ahead-- == 0) grid_dep_wait();   // the MMAs wait for the previous kernel: its time is not this barrier's
-                if (!__all_sync(0xffffffffu, mbar_wait(full_p(ps), pph, abort_flag, p.status, 51) && mbar_wait(empty(gs), ph ^ 1u, abort_flag, p.status, 52))) {
+                if (!__all_sync(0xffffffffu, mbar_wait(full_p(ps), pph, abort_flag, p.status, 51, p.wait_limit) && mbar_wait(empty(gs), ph ^ 1u, abort_flag, p.status, 52, p.wait_limit))) {
                     ok = false;
                     break;
                 }
@@ -238,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
             const int nt = column_tile_of(t, w);
             for (int kb = kb0; kb < kb1; kb += kGroup) {
                 if (ahead-- == 0) grid_dep_wait();   // (as above: the expand warps have emptied kRing groups by then)
-                if (!__all_sync(0xffffffffu, mbar_wait(empty_p(s), ph ^ 1u, abort_flag, p.status, 53))) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(empty_p(s), ph ^ 1u, abort_flag, p.status, 53, p.wait_limit))) { ok = false; break; }
                 if (leader) {
                     // (always a whole box: what lies beyond the weight reads as zeros, a surplus K block is not expanded)
                     mbar_arrive_expect_tx(full_p(s), kGroup * L::kPStageBytes);
@@ -269,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
                 down = 512; right = 256; next_k = 1024; next_row = (int64_t)kLoaderWarps * p.Kt * 1024;
             }
             for (int kb = kb0; kb < kb1; kb += kGroup) {
-                if (!__all_sync(0xffffffffu, mbar_wait(empty(s), ph ^ 1u, abort_flag, p.status, 54))) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(empty(s), ph ^ 1u, abort_flag, p.status, 54, p.wait_limit))) { ok = false; break; }
                 uint32_t d0 = sbase + L::x + s * kGroup * kXStageBytes + lw * 1024 + face_dst;
                 for (int j = 0; j < min(kGroup, kb1 - kb); ++j, src += next_k, d0 += kXStageBytes) {
                     const uint16_t *f = src;
@@ -298,11 +300,11 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
         uint32_t ph = 0;
         bool ok = true;
         for (int t = first; ok && t < p.tiles; t += step, ++n) {
-            if (!__all_sync(0xffffffffu, mbar_wait(acc_empty, (uint32_t)((n & 1) ^ 1), abort_flag, p.status, 55))) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(acc_empty, (uint32_t)((n & 1) ^ 1), abort_flag, p.status, 55, p.wait_limit))) { ok = false; break; }
             tc_fence_after_sync();
             const uint32_t idesc = instr_desc_bf16_f32(BN, 0, /*a_mn_major=*/false, /*b_mn_major=*/false) | ((uint32_t)(rows_of(chunk_of(t)) >> 3) << 17);
             for (int kb = kb0; kb < kb1; kb += kGroup) {
-                if (!__all_sync(0xffffffffu, mbar_wait(full(gs), ph, abort_flag, p.status, 56))) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(full(gs), ph, abort_flag, p.status, 56, p.wait_limit))) { ok = false; break; }
                 fence_proxy_async_smem();   // the activations came through the generic proxy
                 tc_fence_after_sync();
                 const uint32_t a_col = tmem_base + (uint32_t)(kACol0 + gs * kGroup * kAColsPerStage);
@@ -338,7 +340,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
             int w;
             const int64_t row_base = (int64_t)chunk * p.chunk_rows, col0 = (int64_t)column_tile_of(t, w) * BN + lane * 4;
             // (the eight warps meet at named barriers below: they go on together or not at all)
-            int good = mbar_wait(acc_full, (uint32_t)(n & 1), abort_flag, p.status, 57) ? 1 : 0;
+            int good = mbar_wait(acc_full, (uint32_t)(n & 1), abort_flag, p.status, 57, p.wait_limit) ? 1 : 0;
             asm volatile(
                 "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %0, 0;\n\tbarrier.cta.red.and.pred q, 1, %1, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
                 : "+r"(good)
@@ -522,6 +524,7 @@ int32_t launch_matmul_rows(const void *a, int count, const void *const *w, int w
     p.a_row_major = (flags & TTB_MM_A_ROW_MAJOR) != 0;
     p.out_row_major = (flags & TTB_MM_OUT_ROW_MAJOR) != 0;
     p.status = status;
+    p.wait_limit = barrier_limit_cycles();
     p.weights = count;
     int64_t tiles = 0;
     for (int j = 0; j < count; ++j) {
