@@ -173,14 +173,20 @@ int32_t ttb_unpack_bfp(const void *src_dev, int32_t fmt, void *dst_dev, int32_t 
  * per-output-tile arrival counters that must be zero when the kernel starts: ttb_matmul clears them with a
  * memset on `stream` unless TTB_MM_WORKSPACE_ZEROED is given. */
 int64_t ttb_matmul_workspace_bytes(int32_t w_dtype, int64_t batch, int64_t M, int64_t K, int64_t N, int32_t flags);
-/* Which block-float kernels ttb_matmul uses for a shape (no GPU needed): out[0] = launches (0: none of them, always so for bf16 weights;
- * else tensor-core launches over consecutive row ranges), then per launch its row count and 1 for the prefill kernel, 0
- * for a decode kernel - for as many launches as `out` has room for (out_len >= 5). Decode kernels take up to 256 rows and
- * any N that is a multiple of 32 (blocks of two tile rows when the row count is a multiple of 64 and N a multiple of 128,
- * else of one); the prefill kernel multiples of 128 rows from 512 up with N a multiple of 128; other row counts are served
- * as two ranges, and large row counts with an N the prefill kernel does not take as up to 16 decode launches of 256 rows.
- * This is the plan of fp32 results. bf16 results of 64 rows and more are mostly computed by one kernel for any row and column
- * count instead (csrc/matmul_rows.cu, which needs no workspace; the rule is rows_kernel_takes in csrc/matmul.cu). */
+/* Which kernel computes a call of ttb_matmul (no GPU needed; the answer without one is a B200's): one of these, or a negative
+ * TTB_E_* for sizes, types or flags that ttb_matmul refuses. */
+#define TTB_KERNEL_GENERIC 0 /* CUDA cores, any shape */
+#define TTB_KERNEL_RANGES 1  /* decode and prefill kernels over row ranges: ttb_matmul_plan has them */
+#define TTB_KERNEL_ROWS 2    /* block-float weights, bfloat16 results, any row and column count: csrc/matmul_rows.cu */
+#define TTB_KERNEL_BF16 3    /* bfloat16 weights: csrc/matmul_bf16.cu */
+int32_t ttb_matmul_kernel(int32_t w_dtype, int32_t out_dtype, int64_t batch, int64_t M, int64_t K, int64_t N, int32_t flags);
+/* The row ranges of TTB_KERNEL_RANGES (no GPU needed): out[0] = launches (0: the decode and prefill kernels do not take the shape), then
+ * per launch its row count and 1 for the prefill kernel, 0 for a decode kernel - for as many launches as `out` has room for
+ * (out_len >= 5). Decode kernels take up to 256 rows and any N that is a multiple of 32 (blocks of two tile rows when the row
+ * count is a multiple of 64 and N a multiple of 128, else of one); the prefill kernel multiples of 128 rows from 512 up with N a
+ * multiple of 128; other row counts are served as two ranges, and large row counts with an N the prefill kernel does not take
+ * as up to 16 decode launches of 256 rows. fp32 results of block-float weights always run like this, and so do all results under
+ * TTB_MM_DETERMINISTIC; most bfloat16 results of 64 rows and more run as TTB_KERNEL_ROWS instead, which needs no workspace. */
 int32_t ttb_matmul_plan(int32_t w_dtype, int64_t batch, int64_t M, int64_t K, int64_t N, int32_t flags, int64_t *out, int32_t out_len);
 int32_t ttb_matmul(const void *a_dev, int32_t a_dtype, const void *w_dev, int32_t w_dtype, const void *bias_dev,
                    void *out_dev, int32_t out_dtype, int64_t batch, int64_t M, int64_t K, int64_t N,

@@ -16,6 +16,7 @@ MM_A_ROW_MAJOR, MM_OUT_ROW_MAJOR, MM_FORCE_GENERIC, MM_WORKSPACE_ZEROED, MM_DECO
 MM_WEIGHTS_RESIDENT = 64
 MM_DECODE_SMEM_OPERAND = 128
 MM_GATED = 256
+KERNEL_GENERIC, KERNEL_RANGES, KERNEL_ROWS, KERNEL_BF16 = 0, 1, 2, 3
 TILE_BYTES = {BFLOAT8_B: 1088, BFLOAT4_B: 576}
 
 _vp, _i32, _i64, _sz = ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_size_t
@@ -47,6 +48,7 @@ _SIGS = {
     "ttb_pack_bfp": (_i32, [_vp, _i32, _vp, _i32, _i64, _i64, _i64, _i32, _i32, _vp]),
     "ttb_unpack_bfp": (_i32, [_vp, _i32, _vp, _i32, _i64, _i64, _i64, _i32, _i32, _vp]),
     "ttb_matmul_workspace_bytes": (_i64, [_i32, _i64, _i64, _i64, _i64, _i32]),
+    "ttb_matmul_kernel": (_i32, [_i32, _i32, _i64, _i64, _i64, _i64, _i32]),
     "ttb_matmul_plan": (_i32, [_i32, _i64, _i64, _i64, _i64, _i32, _vp, _i32]),
     "ttb_matmul": (_i32, [_vp, _i32, _vp, _i32, _vp, _vp, _i32, _i64, _i64, _i64, _i64, _i32, _i32, _vp, _i64, _vp]),
     "ttb_bmm": (_i32, [_vp, _i32, _vp, _i32, _vp, _i32, _i64, _i64, _i64, _i64, _vp]),

@@ -30,8 +30,13 @@ def build_fake(directory):
 
 
 @pytest.fixture(scope="module")
-def fake(tmp_path_factory):
-    lib = cabi.Lib(build_fake(str(tmp_path_factory.mktemp("fake"))))
+def fake_so(tmp_path_factory):
+    return build_fake(str(tmp_path_factory.mktemp("fake")))
+
+
+@pytest.fixture(scope="module")
+def fake(fake_so):
+    lib = cabi.Lib(fake_so)
     lib.cdll.fake_log.restype = ctypes.c_char_p
     return lib
 
@@ -112,7 +117,7 @@ def test_a_thread_that_cannot_be_made_is_done_without(fake, failing):
 
 
 @pytest.mark.parametrize("w_dtype", [cabi.BFLOAT16, cabi.BFLOAT8_B, cabi.BFLOAT4_B])
-def test_first_calls_of_several_threads_set_a_kernel_up_once(tmp_path, w_dtype):
+def test_first_calls_of_several_threads_set_a_kernel_up_once(fake_so, w_dtype):
     """The launch reads what the set-up of its device counted: a second thread waits until that is there. (A process of its own: the
     set-up is done once.)"""
     code = """if True:
@@ -131,6 +136,36 @@ def test_first_calls_of_several_threads_set_a_kernel_up_once(tmp_path, w_dtype):
         log = lib.cdll.fake_log().decode().split()
         assert codes == [0] * 4 and len(log) == 4 and len(set(log)) == 1, (codes, log)
         print(lib.cdll.fake_most_configured())
-    """ % (os.path.join(cabi.ROOT, "tests"), build_fake(str(tmp_path)), w_dtype)
+    """ % (os.path.join(cabi.ROOT, "tests"), fake_so, w_dtype)
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.strip() == "1", r.stdout + r.stderr
+
+
+KERNEL_NAMES = {cabi.KERNEL_GENERIC: "matmul_generic_kernel", cabi.KERNEL_ROWS: "matmul_rows_kernel", cabi.KERNEL_BF16: "matmul_bf16_kernel"}
+
+
+@pytest.mark.parametrize("out_dtype", [cabi.BFLOAT16, cabi.FLOAT32])
+@pytest.mark.parametrize("w_dtype", [cabi.BFLOAT16, cabi.BFLOAT8_B, cabi.BFLOAT4_B])
+@pytest.mark.parametrize("flags", [0, cabi.MM_DETERMINISTIC, cabi.MM_FORCE_GENERIC])
+def test_matmul_kernel_names_the_kernel_that_is_launched(fake, w_dtype, out_dtype, flags):
+    """ttb_matmul_kernel against the launches that ttb_matmul makes, and the launches of row ranges against ttb_matmul_plan."""
+    seen = set()
+    for M in (32, 64, 96, 256, 320, 512, 544, 2048):
+        for K, N in ((32, 96), (512, 512), (1024, 4672), (4096, 4096), (8192, 9472)):
+            kind = fake.cdll.ttb_matmul_kernel(w_dtype, out_dtype, 1, M, K, N, flags)
+            fake.cdll.fake_log()
+            rc = fake.cdll.ttb_matmul(4096, cabi.BFLOAT16, 8192, w_dtype, None, 1 << 20, out_dtype, 1, M, K, N, 0, flags | cabi.MM_WORKSPACE_ZEROED, 1 << 21, 1 << 40, None)
+            log = fake.cdll.fake_log().decode().split()
+            assert rc == 0 and log, (M, K, N, rc)
+            if kind == cabi.KERNEL_RANGES:
+                plan = (ctypes.c_int64 * 33)()
+                assert fake.cdll.ttb_matmul_plan(w_dtype, 1, M, K, N, flags, plan, 33) == 0
+                decode = sum("matmul_decode" in k for k in log)
+                assert decode == list(plan)[2:2 + 2 * plan[0]:2].count(0) and not any(n in k for k in log for n in KERNEL_NAMES.values()), (M, K, N, log)
+            else:
+                assert all(KERNEL_NAMES[kind] in k for k in log), (M, K, N, kind, log)
+            seen.add(kind)
+    block_float = {cabi.KERNEL_RANGES, cabi.KERNEL_ROWS} if out_dtype == cabi.BFLOAT16 and not flags else {cabi.KERNEL_RANGES}
+    bf16 = {cabi.KERNEL_BF16} if out_dtype == cabi.BFLOAT16 else {cabi.KERNEL_BF16, cabi.KERNEL_GENERIC}
+    assert seen == ({cabi.KERNEL_GENERIC} if flags & cabi.MM_FORCE_GENERIC else bf16 if w_dtype == cabi.BFLOAT16 else block_float)
+    assert fake.cdll.ttb_matmul_kernel(w_dtype, out_dtype, 1, 32, 48, 64, flags) == -1

@@ -126,6 +126,15 @@ int plan_rows(int w_dtype, int64_t rows, int64_t K, int64_t N, RowChunk (&out)[k
     return 0;
 }
 
+// The kernel of a call whose arguments are valid.
+int kernel_of(int w_dtype, int out_dtype, int64_t rows, int64_t K, int64_t N, int flags) {
+    if (flags & TTB_MM_FORCE_GENERIC) return TTB_KERNEL_GENERIC;
+    if (w_dtype == TTB_BFLOAT16) return bf16_on_tensor_cores(out_dtype, K) && rows / 32 <= 65535 ? TTB_KERNEL_BF16 : TTB_KERNEL_GENERIC;
+    if (rows_kernel_takes(w_dtype, out_dtype, rows, K, N, flags)) return TTB_KERNEL_ROWS;
+    RowChunk chunks[kMaxRowChunks];
+    return plan_rows(w_dtype, rows, K, N, chunks) ? TTB_KERNEL_RANGES : TTB_KERNEL_GENERIC;
+}
+
 }  // namespace
 }  // namespace ttb
 
@@ -146,8 +155,14 @@ int64_t ttb_matmul_workspace_bytes(int32_t w_dtype, int64_t batch, int64_t M, in
     return bytes;
 }
 
-/* Which block-float kernels ttb_matmul would use: out[0] = launches (0: none of them - the shape-generic CUDA-core kernel, or for
- * bfloat16 weights usually the kernel of matmul_bf16.cu; fp32 results, see rows_kernel_takes), then per launch its rows and 1 for the prefill kernel, 0 for a decode kernel - for as many launches as `out` has room for (at least two). */
+int32_t ttb_matmul_kernel(int32_t w_dtype, int32_t out_dtype, int64_t batch, int64_t M, int64_t K, int64_t N, int32_t flags) {
+    const void *const any = reinterpret_cast<const void *>(uintptr_t(256));   // (no tensors: their checks pass)
+    if (int32_t rc = validate(any, TTB_BFLOAT16, any, w_dtype, const_cast<void *>(any), out_dtype, batch, M, K, N, TTB_ACT_NONE)) return rc;
+    return kernel_of(w_dtype, out_dtype, batch * M, K, N, flags);
+}
+
+/* The row ranges of TTB_KERNEL_RANGES: out[0] = launches (0: the decode and prefill kernels do not take the shape), then per launch
+ * its rows and 1 for the prefill kernel, 0 for a decode kernel - for as many launches as `out` has room for (at least two). */
 int32_t ttb_matmul_plan(int32_t w_dtype, int64_t batch, int64_t M, int64_t K, int64_t N, int32_t flags, int64_t *out, int32_t out_len) {
     if (!out || out_len < 5) return fail(TTB_E_INVALID, "ttb_matmul_plan: needs room for 5 values");
     RowChunk chunks[kMaxRowChunks];
@@ -166,27 +181,20 @@ int32_t ttb_matmul(const void *a, int32_t a_dtype, const void *w, int32_t w_dtyp
     if (int32_t rc = validate(a, a_dtype, w, w_dtype, out, out_dtype, batch, M, K, N, act)) return rc;
     const int64_t rows = batch * M;  // tiled [batch, M, K] with M % 32 == 0 is the same buffer as tiled [batch*M, K]
     auto s = (cudaStream_t)stream;
-    if (w_dtype == TTB_BFLOAT16 && !(flags & TTB_MM_FORCE_GENERIC) && bf16_on_tensor_cores(out_dtype, K) && rows / 32 <= 65535) {
-        int *status = nullptr;
-        if (int32_t rc = status_word_address(&status)) return rc;
-        return launch_matmul_bf16(a, w, bias, out, out_dtype, 1, rows, K, N, act, flags, status, s);
-    }
-    if (rows_kernel_takes(w_dtype, out_dtype, rows, K, N, flags)) {
-        int *status = nullptr;
-        if (int32_t rc = status_word_address(&status)) return rc;
-        return launch_matmul_rows(a, 1, &w, w_dtype, &bias, &out, out_dtype, rows, K, &N, act, flags, status, s);
-    }
+    const int kernel = kernel_of(w_dtype, out_dtype, rows, K, N, flags);
+    if (kernel == TTB_KERNEL_GENERIC) return launch_matmul_generic(a, w, w_dtype, bias, out, out_dtype, rows, K, N, act, flags, s);
+    int *status = nullptr;
+    if (int32_t rc = status_word_address(&status)) return rc;
+    if (kernel == TTB_KERNEL_BF16) return launch_matmul_bf16(a, w, bias, out, out_dtype, 1, rows, K, N, act, flags, status, s);
+    if (kernel == TTB_KERNEL_ROWS) return launch_matmul_rows(a, 1, &w, w_dtype, &bias, &out, out_dtype, rows, K, &N, act, flags, status, s);
     RowChunk chunks[kMaxRowChunks];
-    const int n = (flags & TTB_MM_FORCE_GENERIC) ? 0 : plan_rows(w_dtype, rows, K, N, chunks);
-    if (n == 0) return launch_matmul_generic(a, w, w_dtype, bias, out, out_dtype, rows, K, N, act, flags, s);
+    const int n = plan_rows(w_dtype, rows, K, N, chunks);
     const int64_t out_elem = out_dtype == TTB_FLOAT32 ? 4 : 2;
     for (int i = 0; i < n; ++i) {
         const void *ai = static_cast<const uint8_t *>(a) + chunks[i].row0 * K * 2;
         void *oi = static_cast<uint8_t *>(out) + chunks[i].row0 * N * out_elem;
         int32_t rc;
         if (chunks[i].prefill) {
-            int *status = nullptr;
-            if ((rc = status_word_address(&status))) return rc;
             rc = launch_matmul_prefill(ai, w, w_dtype, bias, oi, out_dtype, chunks[i].rows, K, N, act, flags, workspace, workspace_bytes, status, s);
         } else {
             rc = launch_matmul_decode(ai, w, w_dtype, bias, oi, out_dtype, chunks[i].rows, K, N, act, flags, workspace, workspace_bytes,
