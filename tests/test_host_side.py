@@ -169,3 +169,27 @@ def test_matmul_kernel_names_the_kernel_that_is_launched(fake, w_dtype, out_dtyp
     bf16 = {cabi.KERNEL_BF16} if out_dtype == cabi.BFLOAT16 else {cabi.KERNEL_BF16, cabi.KERNEL_GENERIC}
     assert seen == ({cabi.KERNEL_GENERIC} if flags & cabi.MM_FORCE_GENERIC else bf16 if w_dtype == cabi.BFLOAT16 else block_float)
     assert fake.cdll.ttb_matmul_kernel(w_dtype, out_dtype, 1, 32, 48, 64, flags) == -1
+
+
+def kernel(lib, M, K, N, w_dtype=cabi.BFLOAT8_B):
+    return lib.cdll.ttb_matmul_kernel(w_dtype, cabi.BFLOAT16, 1, M, K, N, 0)
+
+
+@pytest.mark.parametrize("w_dtype", [cabi.BFLOAT8_B, cabi.BFLOAT4_B])
+def test_96_to_256_rows_take_the_kernel_that_measured_faster(fake, w_dtype):
+    """Shapes on either side of the line between the decode and the middling-rows kernel, each at least 5 % faster on its side; as one
+    weight, and as several that together have its column tiles."""
+    decode = [(224, 128, 1024), (224, 512, 1024), (160, 256, 1024), (160, 512, 3072), (96, 640, 4096), (96, 1024, 3072), (224, 1024, 2048), (160, 768, 2048),
+              (96, 28672, 256), (96, 12288, 512), (160, 20480, 512), (224, 28672, 384), (256, 20480, 128), (128, 28672, 512), (192, 28672, 256)]
+    rows = [(96, 256, 1024), (160, 256, 4096), (96, 1024, 1024), (192, 512, 1024), (128, 512, 128), (224, 512, 3072), (160, 1536, 512), (96, 512, 6144),
+            (96, 8192, 512), (128, 12288, 256), (160, 28672, 768), (256, 12288, 256), (96, 28672, 1536), (224, 20480, 512), (256, 4096, 128)]
+    for want, shapes in ((cabi.KERNEL_RANGES, decode), (cabi.KERNEL_ROWS, rows)):
+        for M, K, N in shapes:
+            assert kernel(fake, M, K, N, w_dtype) == want, (M, K, N)
+            Ns = (N // 2, N - N // 2) if N % 256 == 0 else (N,)
+            P = lambda at: (ctypes.c_void_p * len(Ns))(*[at + (j << 30) for j in range(len(Ns))])   # noqa: E731
+            fake.cdll.fake_log()
+            fake.check(fake.cdll.ttb_matmul_multi(4096, cabi.BFLOAT16, len(Ns), P(1 << 34), w_dtype, None, P(1 << 38), cabi.BFLOAT16, 1, M, K,
+                                                  (ctypes.c_int64 * len(Ns))(*Ns), 0, cabi.MM_WORKSPACE_ZEROED, 1 << 40, 1 << 40, None, None, None))
+            log = fake.cdll.fake_log().decode().split()
+            assert log and all(("matmul_decode" if want == cabi.KERNEL_RANGES else "matmul_rows") in k for k in log), (M, K, Ns, log)

@@ -60,7 +60,7 @@ def test_against_64_bits(ttb, fmt, M, K, N):
 
 
 @pytest.mark.parametrize("fmt", [cabi.BFLOAT8_B, cabi.BFLOAT4_B])
-@pytest.mark.parametrize("M,K,Ns", [(96, 512, (512, 96, 160)), (128, 1024, (1024, 128)), (256, 288, (96, 4672, 32, 4096))])
+@pytest.mark.parametrize("M,K,Ns", [(96, 512, (512, 96, 160)), (96, 768, (512, 96, 160)), (128, 1024, (1024, 128)), (256, 288, (96, 4672, 32, 4096))])
 def test_several_weights_in_one_launch(ttb, fmt, M, K, Ns):
     import ctypes
     import torch

@@ -11,6 +11,7 @@ int32_t launch_bmm_generic(const void *a, const void *w, int w_dtype, void *out,
 int32_t launch_matmul_bf16(const void *a, const void *w, const void *bias, void *out, int out_dtype, int64_t batch, int64_t rows, int64_t K,
                            int64_t N, int act, int flags, int *status, cudaStream_t stream);
 bool decode_supported(int w_dtype, int64_t rows, int64_t K, int64_t N);
+bool decode_is_faster(int64_t rows, int64_t K, int64_t tiles, bool ragged);
 int64_t decode_workspace_bytes(int64_t rows, int64_t K, int64_t N, bool smem_operand);
 int32_t launch_matmul_decode(const void *a, const void *w, int w_dtype, const void *bias, void *out, int out_dtype,
                              int64_t rows, int64_t K, int64_t N, int act, int flags, void *workspace,
@@ -64,7 +65,8 @@ bool bf16_on_tensor_cores(int out_dtype, int64_t K) { return out_dtype == TTB_BF
 
 // bfloat16 results that the kernel of matmul_rows.cu takes, whole and whatever the column count (fp32 results keep the row ranges
 // below, whose shorter chains of additions bring them closer to 64 bits). Three lines, with both sides measured (us):
-//  * 96 rows and more: 96 x 4096 x 4096 17.0 with the decode kernel, 13.2 here; 128 x 4096 x 14336 bfloat4_b 46.2 / 28.4;
+//  * 96 rows and more, except where the decode kernel is faster (decode_is_faster): 96 x 4096 x 4096 16.0 there, 12.0 here; 128 x
+//    4096 x 14336 bfloat4_b 46.2 / 28.4; above 256 rows, two launches and more there, always: 288 rows and up 0.28 to 0.78 of it;
 //  * 64 rows while its 128-column tiles number at most half the SMs and their K range can be shared: 64 x 8192 x 8192 35.7 /
 //    27.2, 64 x 4096 x 1024 14.9 / 8.9, but 64 x 4096 x 14336 (112 tiles) 21.1 / 26.2, and a 64-row layer with a down projection of
 //    K = 21504 took 185 / 195;
@@ -79,6 +81,7 @@ bool rows_kernel_takes(int w_dtype, int out_dtype, int64_t rows, int64_t K, int6
     constexpr int64_t kSms = 148;
     if (rows == 64) return (N + 127) / 128 * 2 <= kSms && K <= 8192;
     if (rows < 96) return false;
+    if (rows <= 256) return !(decode_supported(w_dtype, rows, K, N) && decode_is_faster(rows, K, (N + 127) / 128, N % 128 != 0));
     if (!prefill_supported(w_dtype, rows, K, N)) return true;
     const int64_t blocks = rows * N / 65536;
     const bool whole_rounds = w_dtype == TTB_BFLOAT8_B && blocks >= 5 * kSms && blocks % kSms * 4 < kSms;

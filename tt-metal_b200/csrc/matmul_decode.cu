@@ -83,7 +83,7 @@ struct StreamPlan {
 };
 // One persistent block per multiprocessor of the current device (read once per process; 148, a B200's count, where no device
 // can be asked - the plan and workspace queries also work without a GPU).
-static int stream_blocks() {
+int stream_blocks() {
     static int cached = 0;
     if (cached == 0) {
         int dev = 0, sms = 0;
@@ -170,6 +170,27 @@ bool decode_supported_multi(int w_dtype, int64_t rows, int64_t K, int nprob, con
         tiles += tiles128(N[j]);
     }
     return tiles * (rows / 32) <= kSyncInt0;
+}
+
+// 96 to 256 rows: whether the decode kernel is the faster one for weights of `tiles` 128-column tiles that share an activation, the
+// other being the kernel of matmul_rows.cu, which expands a weight once for all rows but lets at most eight blocks share a
+// tile's K range. Two corners, from timings of both (us, decode / rows kernel, bfloat8_b; bfloat4_b differs by a few percent):
+//  * blocks of one tile row, all of them running at once, and so short a K range that the larger block's start-up counts:
+//    224 x 512 x 1024 5.6 / 6.8, 160 x 256 x 1024 5.1 / 5.7, 160 x 512 x 3072 6.6 / 7.2, 96 x 640 x 4096 6.7 / 7.6, 96 x 1024 x 3072
+//    7.3 / 7.8, 224 x 1024 x 2048 7.9 / 8.6, but 96 x 256 x 1024 5.3 / 4.8, 160 x 256 x 4096 7.2 / 5.8, 96 x 1024 x 1024 6.8 / 5.8,
+//    160 x 1536 x 1024 8.0 / 7.7, and with two tile rows per block 192 x 512 x 1024 7.6 / 6.6;
+//  * few tiles of a long K range, which eight blocks each do not spread over the chip: 96 x 28672 x 256 12.0 / 21.9, 96 x 12288 x
+//    512 11.6 / 12.3, 256 x 20480 x 128 15.2 / 18.7, but 96 x 8192 x 512 10.4 / 9.8, 128 x 12288 x 256 14.5 / 12.1, 160 x 28672 x 768
+//    27.2 / 24.1. There the decode kernel takes 8.5 us (13.2 with two tile rows per block) + 0.65 (0.8) ns for each K block of
+//    each of its tiles, the other 3.3 us + 12.5 ns per row + 19 ns per K block + 190 ns per tile.
+bool decode_is_faster(int64_t rows, int64_t K, int64_t tiles, bool ragged) {
+    const bool one_row = decode_rows_per_block(rows, false, ragged) == 32;
+    const int64_t blocks = tiles * (rows / (one_row ? 32 : 64)), kb = K / BK;
+    if (one_row && kb <= 32 && blocks <= (rows >= 160 && kb >= 16 ? 120 : 96) && (kb <= (rows >= 160 ? 24 : 20) ? rows >= 160 || kb >= 16 : blocks >= 40))
+        return true;
+    if (tiles > 8 || kb < 256) return false;
+    const double decode = (one_row ? 8500.0 : 13200.0) + (one_row ? 0.65 : 0.8) * (double)(blocks * kb);
+    return decode < 3300.0 + 12.5 * (double)rows + 19.0 * (double)kb + 190.0 * (double)tiles;
 }
 
 // Accumulate mode needs rows * (sum of N) fp32 inside the fixed 16 MiB region; larger outputs use ordered mode.
@@ -545,10 +566,13 @@ extern "C" int32_t ttb_matmul_multi(const void *a, int32_t a_dtype, int32_t coun
     if (batch <= 0 || M <= 0 || M % 32) return fail(TTB_E_INVALID, "ttb_matmul_multi: batch, M, K must be positive and M, K multiples of 32");
     const int64_t rows = batch * M;
     if (int32_t rc = validate_multi("ttb_matmul_multi", a, a_dtype, count, w, w_dtype, out, out_dtype, rows, K, N, act, flags, gather, wait)) return rc;
-    // bfloat16 results of 96 rows and more, of one rank and not gated: the kernel that expands a weight once for all its rows (us
-    // before / now: 96 x 4096 x [4096, 1024, 1024] 19.5 / 18.5, 128 rows 21.5 / 18.6, 256 rows 39.9 / 24.6, 128 x 8192 x [28672,
-    // 28672] 270 / 155).
-    if (rows >= 96 && out_dtype == TTB_BFLOAT16 && !gather && !wait && !(flags & (TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_GATED | TTB_MM_DETERMINISTIC))) {
+    // bfloat16 results of 96 rows and more, of one rank and not gated, except where the decode kernel is faster: the kernel that
+    // expands a weight once for all its rows (us, decode / rows kernel: 96 x 4096 x [4096, 1024, 1024] 17.5 / 16.5, 128 rows 21.0 /
+    // 16.9, 256 rows 38.3 / 22.6, 128 x 8192 x [28672, 28672] 270 / 153; 160 x 512 x [1024, 256, 256] 5.7 / 6.7 stays).
+    int64_t tiles = 0;
+    for (int j = 0; j < count; ++j) tiles += tiles128(N[j]);
+    if (rows >= 96 && out_dtype == TTB_BFLOAT16 && !gather && !wait && !(flags & (TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_GATED | TTB_MM_DETERMINISTIC)) &&
+        !decode_is_faster(rows, K, tiles, any_ragged(count, N))) {
         int *status = nullptr;
         if (int32_t rc = status_word_address(&status)) return rc;
         return launch_matmul_rows(a, count, w, w_dtype, bias, out, out_dtype, rows, K, N, act, flags, status, (cudaStream_t)stream);
