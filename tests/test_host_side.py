@@ -193,3 +193,19 @@ def test_96_to_256_rows_take_the_kernel_that_measured_faster(fake, w_dtype):
                                                   (ctypes.c_int64 * len(Ns))(*Ns), 0, cabi.MM_WORKSPACE_ZEROED, 1 << 40, 1 << 40, None, None, None))
             log = fake.cdll.fake_log().decode().split()
             assert log and all(("matmul_decode" if want == cabi.KERNEL_RANGES else "matmul_rows") in k for k in log), (M, K, Ns, log)
+
+
+@pytest.mark.parametrize("shape,w_dtype,prefill", [
+    # short K ranges: nearly full last rounds, then broken ones and blocks that are not 256 x 256
+    ((1024, 256, 9472), cabi.BFLOAT8_B, True), ((1024, 1024, 18944), cabi.BFLOAT8_B, True), ((1024, 512, 16384), cabi.BFLOAT4_B, True),
+    ((2048, 512, 28672), cabi.BFLOAT4_B, True), ((1536, 512, 28672), cabi.BFLOAT8_B, True), ((768, 512, 12544), cabi.BFLOAT4_B, True),
+    ((512, 1024, 28416), cabi.BFLOAT8_B, False), ((640, 1024, 14336), cabi.BFLOAT4_B, False), ((512, 1024, 14208), cabi.BFLOAT8_B, False),
+    ((1024, 2048, 9472), cabi.BFLOAT8_B, False), ((2048, 512, 16384), cabi.BFLOAT8_B, False), ((512, 512, 9472), cabi.BFLOAT8_B, False),
+    # long ones
+    ((1024, 8192, 18944), cabi.BFLOAT8_B, True), ((1024, 8192, 28416), cabi.BFLOAT8_B, True), ((1024, 28672, 8192), cabi.BFLOAT8_B, True),
+    ((2048, 8192, 28672), cabi.BFLOAT8_B, True), ((2048, 12288, 18944), cabi.BFLOAT4_B, True),
+    ((2048, 8192, 4096), cabi.BFLOAT8_B, False), ((2048, 8192, 8192), cabi.BFLOAT8_B, False), ((1024, 8192, 18944), cabi.BFLOAT4_B, False),
+    ((2048, 4096, 28672), cabi.BFLOAT8_B, False), ((2048, 8192, 28672), cabi.BFLOAT4_B, False), ((1024, 4096, 9472), cabi.BFLOAT8_B, False)])
+def test_512_rows_and_more_take_the_kernel_that_measured_faster(fake, shape, w_dtype, prefill):
+    """Shapes on either side of the line between the prefill and the middling-rows kernel."""
+    assert kernel(fake, *shape, w_dtype) == (cabi.KERNEL_RANGES if prefill else cabi.KERNEL_ROWS)

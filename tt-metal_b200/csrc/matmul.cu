@@ -12,6 +12,7 @@ int32_t launch_matmul_bf16(const void *a, const void *w, const void *bias, void 
                            int64_t N, int act, int flags, int *status, cudaStream_t stream);
 bool decode_supported(int w_dtype, int64_t rows, int64_t K, int64_t N);
 bool decode_is_faster(int64_t rows, int64_t K, int64_t tiles, bool ragged);
+int stream_blocks();
 int64_t decode_workspace_bytes(int64_t rows, int64_t K, int64_t N, bool smem_operand);
 int32_t launch_matmul_decode(const void *a, const void *w, int w_dtype, const void *bias, void *out, int out_dtype,
                              int64_t rows, int64_t K, int64_t N, int act, int flags, void *workspace,
@@ -63,30 +64,43 @@ int32_t validate(const void *a, int a_dtype, const void *w, int w_dtype, void *o
 // 5.1e-8; at 128: 7.1e-8 against 7.3e-8, and the longer the further ahead).
 bool bf16_on_tensor_cores(int out_dtype, int64_t K) { return out_dtype == TTB_BFLOAT16 || K >= 128; }
 
+// bfloat16 results that the prefill kernel computes faster than the one of matmul_rows.cu: whole 256 x 256 blocks whose last round
+// over the multiprocessors is nearly full (anything broken favours the finer tiles there: us, prefill / rows kernel, 1.5 rounds 512 x
+// 1024 x 28416 55.5 / 45.1, blocks of 128 rows or columns 640 x 1024 x 14336 63 / 39, 512 x 1024 x 14208 41 / 28), and
+//  * a short K range, where a round's fixed part counts: 1.0 round 1024 x 256 x 9472 18.2 / 20.2, 1024 x 1024 x 9472 30.3 / 31.3, 1.7
+//    rounds 1024 x 512 x 16384 40.9 / 44.7, 3.0 rounds 1024 x 768 x 28416 72.9 / 76.5, but 1024 x 2048 x 9472 45.3 / 44.5; at K = 512
+//    from four rounds on with any last one: 4.5 rounds 1536 x 512 x 28672 97.8 / 100.8, 6.05 rounds 2048 x 512 x 28672 129.4 / 133.5,
+//    but 3.5 rounds 2048 x 512 x 16384 78.3 / 74.1;
+//  * a long one, where the chip runs into its power limit and the kernel that moves less data gains: bfloat8_b 2.0 rounds 1024 x 8192 x
+//    18944 265.5 / 274.8, 3.0 rounds 1024 x 6144 x 28416 303.6 / 312.3, 0.9 rounds 1024 x 28672 x 8192 432.8 / 450.5, bfloat4_b 4.0
+//    rounds 2048 x 12288 x 18944 810.7 / 844.0, but bfloat8_b 0.9 rounds 2048 x 8192 x 4096 141.2 / 131.1, 1.7 rounds 2048 x 8192 x 8192
+//    275 / 248, bfloat4_b 2.0 rounds 1024 x 8192 x 18944 281 / 259; with many rounds a small remainder costs little: 6.05 rounds
+//    2048 x 8192 x 28672 860 / 853 to 890, but 2048 x 4096 x 28672 526 / 479.
+bool prefill_is_faster(int w_dtype, int64_t rows, int64_t K, int64_t N) {
+    if (rows % 256 || N % 256) return false;
+    const int64_t sms = stream_blocks(), blocks = rows / 256 * (N / 256), last = (blocks - 1) % sms + 1;
+    const bool full = last * 16 >= sms * 15;
+    if (K <= 1024) return last * 10 >= sms * 7 || (K <= 512 && blocks >= 4 * sms);
+    if (w_dtype == TTB_BFLOAT4_B) return full && K >= 12288;
+    if (K >= 8192) return full || (K >= 12288 && last * 20 >= sms * 17) || (blocks >= 5 * sms && last * 4 < sms);
+    return full && K >= 6144 && blocks > 2 * sms;
+}
+
 // bfloat16 results that the kernel of matmul_rows.cu takes, whole and whatever the column count (fp32 results keep the row ranges
 // below, whose shorter chains of additions bring them closer to 64 bits). Three lines, with both sides measured (us):
 //  * 96 rows and more, except where the decode kernel is faster (decode_is_faster): 96 x 4096 x 4096 16.0 there, 12.0 here; 128 x
 //    4096 x 14336 bfloat4_b 46.2 / 28.4; above 256 rows, two launches and more there, always: 288 rows and up 0.28 to 0.78 of it;
-//  * 64 rows while its 128-column tiles number at most half the SMs and their K range can be shared: 64 x 8192 x 8192 35.7 /
-//    27.2, 64 x 4096 x 1024 14.9 / 8.9, but 64 x 4096 x 14336 (112 tiles) 21.1 / 26.2, and a 64-row layer with a down projection of
-//    K = 21504 took 185 / 195;
-//  * where the prefill kernel applies, it keeps two kinds of shapes: bfloat8_b weights whose 256 x 256 blocks come to five or more
-//    whole rounds with little left over (2048 x 8192 x 28672, 6.05 rounds: 862 there, 890 here; broken rounds favour the finer
-//    tiles here: 1.7 rounds, 2048 x 8192 x 8192, 268 / 239; 3.5 rounds, 2048 x 2048 x 16384, 168 / 147; bfloat4_b 6.05 rounds 932 /
-//    835), and single, nearly full rounds of a short K range (1024 x 2048 x 8192 bfloat4_b 45.2 / 46.0, but 2048 x 4096 x 4096
-//    81.2 / 74.0); 512 x 4096 x 4096 (32 blocks) 74.8 / 24.0.
+//  * 64 rows while its 128-column tiles number at most half the SMs and their K range can be shared: 64 x 8192 x 8192 34.2 /
+//    27.1, 64 x 4096 x 1024 14.2 / 8.0, 64 x 8192 x 9472 (74 tiles) 34.1 / 28.1, but 64 x 8192 x 9600 (75 tiles) 34.0 / 46.0; up to a K
+//    at which that is so for any column count (64 x 20480 x 512 15.8 / 17.0);
+//  * where the prefill kernel applies, except for the shapes that it keeps.
 bool rows_kernel_takes(int w_dtype, int out_dtype, int64_t rows, int64_t K, int64_t N, int flags) {
     // (under TTB_MM_DETERMINISTIC a call gives the bytes of the same stage of a sequence, which the decode kernel computes)
     if (w_dtype == TTB_BFLOAT16 || out_dtype != TTB_BFLOAT16 || (flags & (TTB_MM_FORCE_GENERIC | TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_DETERMINISTIC))) return false;
-    constexpr int64_t kSms = 148;
-    if (rows == 64) return (N + 127) / 128 * 2 <= kSms && K <= 8192;
+    if (rows == 64) return (N + 127) / 128 * 2 <= stream_blocks() && K <= 8192;
     if (rows < 96) return false;
     if (rows <= 256) return !(decode_supported(w_dtype, rows, K, N) && decode_is_faster(rows, K, (N + 127) / 128, N % 128 != 0));
-    if (!prefill_supported(w_dtype, rows, K, N)) return true;
-    const int64_t blocks = rows * N / 65536;
-    const bool whole_rounds = w_dtype == TTB_BFLOAT8_B && blocks >= 5 * kSms && blocks % kSms * 4 < kSms;
-    const bool one_short_round = blocks * 4 >= kSms * 3 && blocks <= kSms && K <= 2048;
-    return !(whole_rounds || one_short_round);
+    return !(prefill_supported(w_dtype, rows, K, N) && prefill_is_faster(w_dtype, rows, K, N));
 }
 
 // Row ranges of one matmul and the tensor-core kernel that takes each: the decode kernels serve up to 256 rows, the prefill
