@@ -166,7 +166,7 @@ def test_matmul_kernel_names_the_kernel_that_is_launched(fake, w_dtype, out_dtyp
                 assert all(KERNEL_NAMES[kind] in k for k in log), (M, K, N, kind, log)
             seen.add(kind)
     block_float = {cabi.KERNEL_RANGES, cabi.KERNEL_ROWS} if out_dtype == cabi.BFLOAT16 and not flags else {cabi.KERNEL_RANGES}
-    bf16 = {cabi.KERNEL_BF16} if out_dtype == cabi.BFLOAT16 else {cabi.KERNEL_BF16, cabi.KERNEL_GENERIC}
+    bf16 = {cabi.KERNEL_BF16, cabi.KERNEL_GENERIC}
     assert seen == ({cabi.KERNEL_GENERIC} if flags & cabi.MM_FORCE_GENERIC else bf16 if w_dtype == cabi.BFLOAT16 else block_float)
     assert fake.cdll.ttb_matmul_kernel(w_dtype, out_dtype, 1, 32, 48, 64, flags) == -1
 
@@ -209,3 +209,16 @@ def test_96_to_256_rows_take_the_kernel_that_measured_faster(fake, w_dtype):
 def test_512_rows_and_more_take_the_kernel_that_measured_faster(fake, shape, w_dtype, prefill):
     """Shapes on either side of the line between the prefill and the middling-rows kernel."""
     assert kernel(fake, *shape, w_dtype) == (cabi.KERNEL_RANGES if prefill else cabi.KERNEL_ROWS)
+
+
+@pytest.mark.parametrize("batch,M,K,N,tensor_cores", [
+    (1, 32, 32, 32, False), (1, 128, 32, 512, False), (1, 512, 32, 512, False), (1000, 32, 32, 32, False), (4000, 32, 64, 32, False), (32, 64, 32, 64, False),
+    (1, 1024, 32, 1024, True), (32, 128, 32, 128, True), (500, 32, 64, 32, True), (1, 32, 64, 1024, True), (1000, 32, 64, 128, True), (1, 32, 96, 32, True)])
+def test_small_bfloat16_products_take_the_kernel_that_measured_faster(fake, batch, M, K, N, tensor_cores):
+    """Batched (ttb_bmm) and, for one matrix, also as a linear: shapes on either side of the line between CUDA and tensor cores."""
+    fake.cdll.fake_log()
+    fake.check(fake.cdll.ttb_bmm(4096, cabi.BFLOAT16, 8192, cabi.BFLOAT16, 16384, cabi.BFLOAT16, batch, M, K, N, None))
+    log = fake.cdll.fake_log().decode().split()
+    assert len(log) == 1 and ("matmul_bf16_kernel" in log[0]) == tensor_cores, log
+    if batch == 1:
+        assert kernel(fake, M, K, N, cabi.BFLOAT16) == (cabi.KERNEL_BF16 if tensor_cores else cabi.KERNEL_GENERIC)

@@ -9,9 +9,9 @@ import cabi
 
 pytestmark = pytest.mark.gpu
 
-# rows, K, N: one tile of each kind; partial row tiles, partial column tiles, a last K stage of 32; K ranges shared by clusters
+# rows, K, N: one tile of each kind (CUDA cores, then many tiles of it); partial row tiles, partial column tiles, a last K stage of 32; K ranges shared by clusters
 # of 8, 4 and 2 blocks; more tiles than SMs
-SHAPES = [(32, 32, 32), (64, 96, 160), (160, 64, 96), (96, 2048, 96), (128, 1056, 1024), (512, 544, 1120), (1312, 160, 2080)]
+SHAPES = [(32, 32, 32), (1024, 32, 1056), (64, 96, 160), (160, 64, 96), (96, 2048, 96), (128, 1056, 1024), (512, 544, 1120), (1312, 160, 2080)]
 
 
 def expect(x, w, bias, act):

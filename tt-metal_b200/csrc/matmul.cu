@@ -59,10 +59,20 @@ int32_t validate(const void *a, int a_dtype, const void *w, int w_dtype, void *o
     return TTB_OK;
 }
 
-// bfloat16 weights: the tensor-core kernel, except for fp32 results of fewer than 128 products, where its additions (which
-// cut off low bits) come out further from 64 bits than a chain of fused multiply-adds (2-norm at K = 64: 6.5e-8 against
-// 5.1e-8; at 128: 7.1e-8 against 7.3e-8, and the longer the further ahead).
-bool bf16_on_tensor_cores(int out_dtype, int64_t K) { return out_dtype == TTB_BFLOAT16 || K >= 128; }
+// bfloat16 weights: the tensor-core kernel, except for
+//  * fp32 results of fewer than 128 products, where its additions (which cut off low bits) come out further from 64 bits than a
+//    chain of fused multiply-adds (2-norm at K = 64: 6.5e-8 against 5.1e-8; at 128: 7.1e-8 against 7.3e-8, and the longer the
+//    further ahead);
+//  * 32 products of small results, where its start-up or, with many small batch entries, a 128 x 128 tile for each costs more
+//    than the CUDA cores' 32 x 32 tiles (us, CUDA cores / tensor cores: 128 x 32 x 512 2.8 / 3.6, 512 x 32 x 512 3.4 / 3.9, 1000 x [32 x
+//    32 x 32] 7.1 / 10.6, but 1024 x 32 x 1024 7.0 / 4.0, 32 x [128 x 32 x 128] 5.1 / 4.1), and 64 products of many batch entries of one
+//    tile (4000 x [32 x 64 x 32] 32.5 / 35.2, 1000 10.4 / 10.8, but 500 7.1 / 7.0).
+bool bf16_on_tensor_cores(int out_dtype, int64_t batch, int64_t rows, int64_t K, int64_t N) {
+    const int64_t small = batch * (rows / 32) * (N / 32), large = batch * ((rows + 127) / 128) * ((N + 127) / 128);
+    if (K == 32 && small < 300 + large) return false;
+    if (K == 64 && small == large && large >= 1000) return false;
+    return out_dtype == TTB_BFLOAT16 || K >= 128;
+}
 
 // bfloat16 results that the prefill kernel computes faster than the one of matmul_rows.cu: whole 256 x 256 blocks whose last round
 // over the multiprocessors is nearly full (anything broken favours the finer tiles there: us, prefill / rows kernel, 1.5 rounds 512 x
@@ -146,7 +156,7 @@ int plan_rows(int w_dtype, int64_t rows, int64_t K, int64_t N, RowChunk (&out)[k
 // The kernel of a call whose arguments are valid.
 int kernel_of(int w_dtype, int out_dtype, int64_t rows, int64_t K, int64_t N, int flags) {
     if (flags & TTB_MM_FORCE_GENERIC) return TTB_KERNEL_GENERIC;
-    if (w_dtype == TTB_BFLOAT16) return bf16_on_tensor_cores(out_dtype, K) && rows / 32 <= 65535 ? TTB_KERNEL_BF16 : TTB_KERNEL_GENERIC;
+    if (w_dtype == TTB_BFLOAT16) return bf16_on_tensor_cores(out_dtype, 1, rows, K, N) && rows / 32 <= 65535 ? TTB_KERNEL_BF16 : TTB_KERNEL_GENERIC;
     if (rows_kernel_takes(w_dtype, out_dtype, rows, K, N, flags)) return TTB_KERNEL_ROWS;
     RowChunk chunks[kMaxRowChunks];
     return plan_rows(w_dtype, rows, K, N, chunks) ? TTB_KERNEL_RANGES : TTB_KERNEL_GENERIC;
@@ -225,7 +235,7 @@ int32_t ttb_matmul(const void *a, int32_t a_dtype, const void *w, int32_t w_dtyp
 int32_t ttb_bmm(const void *a, int32_t a_dtype, const void *w, int32_t w_dtype, void *out, int32_t out_dtype, int64_t batch, int64_t M,
                 int64_t K, int64_t N, void *stream) {
     if (int32_t rc = validate(a, a_dtype, w, w_dtype, out, out_dtype, batch, M, K, N, TTB_ACT_NONE)) return rc;
-    if (w_dtype == TTB_BFLOAT16 && bf16_on_tensor_cores(out_dtype, K) && M / 32 <= 65535 && batch <= 65535) {
+    if (w_dtype == TTB_BFLOAT16 && bf16_on_tensor_cores(out_dtype, batch, M, K, N) && M / 32 <= 65535 && batch <= 65535) {
         int *status = nullptr;
         if (int32_t rc = status_word_address(&status)) return rc;
         return launch_matmul_bf16(a, w, nullptr, out, out_dtype, batch, M, K, N, TTB_ACT_NONE, 0, status, (cudaStream_t)stream);
