@@ -223,10 +223,14 @@ def test_prefill_kernel_small_shapes(ttb, orc, w_dtype, M, K, N):
     check(ttb.untilize(y, 1, M, N).reshape(M, N), x.float() @ w_ref)
 
 
+@pytest.mark.parametrize("flags", [0, cabi.MM_DETERMINISTIC])
 @pytest.mark.parametrize("act", [cabi.ACT_NONE, cabi.ACT_GELU])
-def test_prefill_kernel_bias_activation_layouts(ttb, orc, act):
+def test_prefill_kernel_bias_activation_layouts(ttb, orc, act, flags):
+    """(A result of a few blocks runs on the middling-rows kernel, under MM_DETERMINISTIC on the prefill kernel.)"""
     import torch
     M, K, N = 512, 128, 256
+    assert ttb.cdll.ttb_matmul_kernel(cabi.BFLOAT8_B, cabi.BFLOAT16, 1, M, K, N, flags) == (cabi.KERNEL_RANGES if flags else cabi.KERNEL_ROWS)
+    assert _plan(ttb, cabi.BFLOAT8_B, M, K, N)[:3] == [1, M, 1]
     x, w_dev, w_ref = make_case(ttb, orc, 43, M, K, N, cabi.BFLOAT8_B)
     bias = vectors.randn(78, (N,), 0.5).bfloat16()
     bias_tile = torch.zeros(32, N, dtype=torch.bfloat16)
@@ -234,15 +238,15 @@ def test_prefill_kernel_bias_activation_layouts(ttb, orc, act):
     b_dev = ttb.tilize(bias_tile.cuda(), 1, 32, N)
     y_ref = act_ref(x.float() @ w_ref + bias.float(), act)
     a = ttb.tilize(x.cuda(), 1, M, K)
-    y = ttb.untilize(ttb.matmul(a, w_dev, cabi.BFLOAT8_B, 1, M, K, N, bias=b_dev, act=act), 1, M, N).reshape(M, N)
+    y = ttb.untilize(ttb.matmul(a, w_dev, cabi.BFLOAT8_B, 1, M, K, N, bias=b_dev, act=act, flags=flags), 1, M, N).reshape(M, N)
     check(y, y_ref)
     y2 = ttb.matmul(x.cuda().contiguous(), w_dev, cabi.BFLOAT8_B, 1, M, K, N, bias=b_dev, act=act,
-                    flags=cabi.MM_A_ROW_MAJOR | cabi.MM_OUT_ROW_MAJOR).reshape(M, N)
+                    flags=flags | cabi.MM_A_ROW_MAJOR | cabi.MM_OUT_ROW_MAJOR).reshape(M, N)
     check(y2, y_ref)
     # batch of four 128-row slabs sharing the weight
     xb = x.reshape(4, 128, K)
     ab = ttb.tilize(xb.cuda(), 4, 128, K)
-    yb = ttb.untilize(ttb.matmul(ab, w_dev, cabi.BFLOAT8_B, 4, 128, K, N, bias=b_dev, act=act), 4, 128, N).reshape(M, N)
+    yb = ttb.untilize(ttb.matmul(ab, w_dev, cabi.BFLOAT8_B, 4, 128, K, N, bias=b_dev, act=act, flags=flags), 4, 128, N).reshape(M, N)
     check(yb, y_ref)
 
 
@@ -352,8 +356,9 @@ def test_overlapped_launches_keep_their_dependencies(ttb, orc, tmem, M):
 @pytest.mark.parametrize("w_dtype", [cabi.BFLOAT8_B, cabi.BFLOAT4_B])
 @pytest.mark.parametrize("M,K,Ns", [(32, 2048, [512, 128, 256]), (64, 1024, [128, 384]), (32, 8192, [1024, 128, 128]), (128, 512, [256, 128]),
                                      (96, 4096, [256, 256, 128, 128])])
-def test_several_weights_in_one_launch(ttb, orc, w_dtype, M, K, Ns):
-    """ttb_matmul_multi: every output equals the single-weight result (same tolerances against the fp32 reference), with
+@pytest.mark.parametrize("flags", [0, cabi.MM_DETERMINISTIC])
+def test_several_weights_in_one_launch(ttb, orc, w_dtype, M, K, Ns, flags):
+    """ttb_matmul_multi (the decode kernel; from 96 rows on the middling-rows kernel unless MM_DETERMINISTIC is asked for): every output equals the single-weight result (same tolerances against the fp32 reference), with
     per-weight bias, a fused activation, and the scratch left clean for the next launch."""
     import ctypes
     import torch
@@ -377,7 +382,7 @@ def test_several_weights_in_one_launch(ttb, orc, w_dtype, M, K, Ns):
     ws = torch.zeros(max(nbytes, 16), dtype=torch.uint8, device="cuda")
     for rep in range(2):
         ttb.check(ttb.cdll.ttb_matmul_multi(a.data_ptr(), cabi.BFLOAT16, n, arr_w, w_dtype, arr_b, arr_o, cabi.BFLOAT16, 1, M, K, arr_n,
-                                            cabi.ACT_SILU, cabi.MM_WORKSPACE_ZEROED | cabi.MM_WEIGHTS_RESIDENT, ws.data_ptr(), nbytes, None, None, None))
+                                            cabi.ACT_SILU, flags | cabi.MM_WORKSPACE_ZEROED | cabi.MM_WEIGHTS_RESIDENT, ws.data_ptr(), nbytes, None, None, None))
         ttb.check(ttb.check_status(None))
         for j, N in enumerate(Ns):
             y_ref = x.float() @ w_refs[j]
@@ -511,16 +516,18 @@ def test_row_counts_between_the_kernels_run_as_two_ranges(ttb, orc, M, kinds):
         check(y.reshape(M, N), torch.relu(x.float().cuda() @ w_ref.cuda()))
 
 
+@pytest.mark.parametrize("kept", [0, cabi.MM_DETERMINISTIC])
 @pytest.mark.parametrize("M,K,N,launches", [(512, 512, 416, 2), (1056, 1024, 4672, 5)])
-def test_large_row_counts_with_a_partial_column_tile_run_as_decode_ranges(ttb, orc, M, K, N, launches):
-    """What the prefill kernel does not take (N not a multiple of 128) runs as decode launches over ranges of 256 rows - not on
-    the CUDA-core kernel - with tiled and with row-major operands, and no byte behind the output is touched."""
+def test_large_row_counts_with_a_partial_column_tile_run_as_decode_ranges(ttb, orc, M, K, N, launches, kept):
+    """What the prefill kernel does not take (N not a multiple of 128) runs as decode launches over ranges of 256 rows where the
+    middling-rows kernel does not take it either (fp32 results, and all under MM_DETERMINISTIC) - not on the CUDA-core kernel - with tiled and with row-major operands, and no byte behind the output is touched."""
     import ctypes
     import torch
     w_dtype = cabi.BFLOAT8_B
     out = (ctypes.c_int64 * 33)()
     assert ttb.cdll.ttb_matmul_plan(w_dtype, 1, M, K, N, 0, out, 33) == 0
     assert out[0] == launches and sum(list(out)[1::2]) == M and not any(list(out)[2::2])
+    assert ttb.cdll.ttb_matmul_kernel(w_dtype, cabi.BFLOAT16, 1, M, K, N, kept) == (cabi.KERNEL_RANGES if kept else cabi.KERNEL_ROWS)
     x, w_dev, w_ref = make_case(ttb, orc, 23, M, K, N, w_dtype)
     ref = torch.relu(x.float().cuda() @ w_ref.cuda())
     for flags in (0, cabi.MM_A_ROW_MAJOR | cabi.MM_OUT_ROW_MAJOR):
@@ -529,7 +536,7 @@ def test_large_row_counts_with_a_partial_column_tile_run_as_decode_ranges(ttb, o
         nbytes = ttb.matmul_workspace_bytes(w_dtype, 1, M, K, N, flags)
         ws = torch.zeros(max(nbytes, 16), dtype=torch.uint8, device="cuda")
         ttb.check(ttb.cdll.ttb_matmul(a.data_ptr(), cabi.BFLOAT16, w_dev.data_ptr(), w_dtype, None, buf.data_ptr(), cabi.BFLOAT16, 1, M, K, N,
-                                      cabi.ACT_RELU, flags | cabi.MM_WORKSPACE_ZEROED, ws.data_ptr(), nbytes, None))
+                                      cabi.ACT_RELU, kept | flags | cabi.MM_WORKSPACE_ZEROED, ws.data_ptr(), nbytes, None))
         ttb.check(ttb.check_status(None))
         assert bool((buf[M * N:] == 7.0).all())
         y = buf[: M * N] if flags else ttb.untilize(buf[: M * N].clone(), 1, M, N)

@@ -23,8 +23,8 @@ def reference(x, w, bias, act):
     return {cabi.ACT_NONE: lambda v: v, cabi.ACT_RELU: torch.relu, cabi.ACT_GELU: torch.nn.functional.gelu, cabi.ACT_SILU: torch.nn.functional.silu}[act](y), mag
 
 
-def close(y, want, mag):
-    bound = 2.0 ** -8 * want.abs() + 2.0 ** -15 * mag
+def close(y, want, mag, K=4096):
+    bound = 2.0 ** -8 * want.abs() + K / 16 * 2.0 ** -23 * mag
     assert bool(((y.double() - want).abs() <= bound).all()), float(((y.double() - want).abs() / bound).max())
 
 
@@ -57,6 +57,31 @@ def test_against_64_bits(ttb, fmt, M, K, N):
         assert bool((buf[:8] == 7.0).all()) and bool((buf[8 + M * N:] == 7.0).all()) and int(ws.count_nonzero()) == 0
         y = out.reshape(M, N) if flags & cabi.MM_OUT_ROW_MAJOR else ttb.untilize(out.clone(), 1, M, N).reshape(M, N)
         close(y, *reference(x, values, bias, act))
+
+
+# long K ranges with and without a cluster, row counts far above one chunk (whole rounds with and without a remainder launch)
+@pytest.mark.parametrize("fmt", [cabi.BFLOAT8_B, cabi.BFLOAT4_B])
+@pytest.mark.parametrize("M,K,N", [(96, 28672, 1152), (320, 12288, 160), (352, 8192, 18976), (1888, 512, 4544), (2048, 2048, 2048), (4096, 288, 1184)])
+def test_long_k_ranges_and_many_rows(ttb, fmt, M, K, N):
+    import torch
+    assert ttb.cdll.ttb_matmul_kernel(fmt, cabi.BFLOAT16, 1, M, K, N, 0) == cabi.KERNEL_ROWS
+    packed, values = weight(ttb, fmt, K, N, 0.02, 5)
+    x = torch.randn(M, K, generator=torch.Generator(device="cuda").manual_seed(6), device="cuda").bfloat16()
+    y = ttb.untilize(ttb.matmul(ttb.tilize(x, 1, M, K), packed, fmt, 1, M, K, N), 1, M, N).reshape(M, N)
+    close(y, *reference(x, values, None, cabi.ACT_NONE), K=K)
+
+
+@pytest.mark.parametrize("fmt", [cabi.BFLOAT8_B, cabi.BFLOAT4_B])
+@pytest.mark.parametrize("M,K,N", [(96, 160, 96), (320, 4096, 160)])
+def test_infinities_and_nan_stay_in_their_rows(ttb, fmt, M, K, N):
+    """Rows share tiles and, with a K range in pieces, partial sums; a non-finite activation reaches its own row only."""
+    import torch
+    packed, values = weight(ttb, fmt, K, N, 0.02, 7)
+    x = torch.randn(M, K, generator=torch.Generator(device="cuda").manual_seed(8), device="cuda").bfloat16()
+    x[5, 33], x[40, 100], x[M - 1, K - 1] = float("inf"), float("nan"), float("-inf")
+    y = ttb.untilize(ttb.matmul(ttb.tilize(x, 1, M, K), packed, fmt, 1, M, K, N), 1, M, N).reshape(M, N)
+    want = x.double() @ values.double()
+    assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isposinf(y), torch.isposinf(want)) and torch.equal(torch.isneginf(y), torch.isneginf(want))
 
 
 @pytest.mark.parametrize("fmt", [cabi.BFLOAT8_B, cabi.BFLOAT4_B])
