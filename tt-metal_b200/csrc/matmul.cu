@@ -83,7 +83,7 @@ bool bf16_on_tensor_cores(int out_dtype, int64_t batch, int64_t rows, int64_t K,
 //    but 3.5 rounds 2048 x 512 x 16384 78.3 / 74.1;
 //  * a long one, where the chip runs into its power limit and the kernel that moves less data gains: bfloat8_b 2.0 rounds 1024 x 8192 x
 //    18944 265.5 / 274.8, 3.0 rounds 1024 x 6144 x 28416 303.6 / 312.3, 0.9 rounds 1024 x 28672 x 8192 432.8 / 450.5, bfloat4_b 4.0
-//    rounds 2048 x 12288 x 18944 810.7 / 844.0, but bfloat8_b 0.9 rounds 2048 x 8192 x 4096 141.2 / 131.1, 1.7 rounds 2048 x 8192 x 8192
+//    rounds 2048 x 12288 x 18944 810.7 / 844.0, 6.0 rounds 2048 x 8192 x 28416 772.8 / 806.4, but bfloat8_b 0.9 rounds 2048 x 8192 x 4096 141.2 / 131.1, 1.7 rounds 2048 x 8192 x 8192
 //    275 / 248, bfloat4_b 2.0 rounds 1024 x 8192 x 18944 281 / 259; with many rounds a small remainder costs little: 6.05 rounds
 //    2048 x 8192 x 28672 860 / 853 to 890, but 2048 x 4096 x 28672 526 / 479.
 bool prefill_is_faster(int w_dtype, int64_t rows, int64_t K, int64_t N) {
@@ -91,7 +91,7 @@ bool prefill_is_faster(int w_dtype, int64_t rows, int64_t K, int64_t N) {
     const int64_t sms = stream_blocks(), blocks = rows / 256 * (N / 256), last = (blocks - 1) % sms + 1;
     const bool full = last * 16 >= sms * 15;
     if (K <= 1024) return last * 10 >= sms * 7 || (K <= 512 && blocks >= 4 * sms);
-    if (w_dtype == TTB_BFLOAT4_B) return full && K >= 12288;
+    if (w_dtype == TTB_BFLOAT4_B) return full && (K >= 12288 || (K >= 8192 && blocks > 5 * sms));
     if (K >= 8192) return full || (K >= 12288 && last * 20 >= sms * 17) || (blocks >= 5 * sms && last * 4 < sms);
     return full && K >= 6144 && blocks > 2 * sms;
 }

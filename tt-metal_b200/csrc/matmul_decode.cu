@@ -181,16 +181,17 @@ bool decode_supported_multi(int w_dtype, int64_t rows, int64_t K, int nprob, con
 //    160 x 1536 x 1024 8.0 / 7.7, and with two tile rows per block 192 x 512 x 1024 7.6 / 6.6;
 //  * few tiles of a long K range, which eight blocks each do not spread over the chip: 96 x 28672 x 256 12.0 / 21.9, 96 x 12288 x
 //    512 11.6 / 12.3, 256 x 20480 x 128 15.2 / 18.7, but 96 x 8192 x 512 10.4 / 9.8, 128 x 12288 x 256 14.5 / 12.1, 160 x 28672 x 768
-//    27.2 / 24.1. There the decode kernel takes 8.5 us (13.2 with two tile rows per block) + 0.65 (0.8) ns for each K block of
-//    each of its tiles, the other 3.3 us + 12.5 ns per row + 19 ns per K block + 190 ns per tile.
+//    27.2 / 24.1. There the decode kernel takes 8.5 us (13.2 with two tile rows per block) + 0.65 (0.68) ns for each K block of
+//    each of its tiles, the other 3.3 us + 12.5 ns per row + 19 ns per K block + 190 ns per tile, and 4 us more for 160 rows and up of
+//    seven tiles and up (192 x 28672 x 1024 29.5 / 31.0).
 bool decode_is_faster(int64_t rows, int64_t K, int64_t tiles, bool ragged) {
     const bool one_row = decode_rows_per_block(rows, false, ragged) == 32;
     const int64_t blocks = tiles * (rows / (one_row ? 32 : 64)), kb = K / BK;
     if (one_row && kb <= 32 && blocks <= (rows >= 160 && kb >= 16 ? 120 : 96) && (kb <= (rows >= 160 ? 24 : 20) ? rows >= 160 || kb >= 16 : blocks >= 40))
         return true;
     if (tiles > 8 || kb < 256) return false;
-    const double decode = (one_row ? 8500.0 : 13200.0) + (one_row ? 0.65 : 0.8) * (double)(blocks * kb);
-    return decode < 3300.0 + 12.5 * (double)rows + 19.0 * (double)kb + 190.0 * (double)tiles;
+    const double decode = (one_row ? 8500.0 : 13200.0) + (one_row ? 0.65 : 0.68) * (double)(blocks * kb);
+    return decode < 3300.0 + 12.5 * (double)rows + 19.0 * (double)kb + 190.0 * (double)tiles + (rows >= 160 && tiles >= 7 ? 4000.0 : 0.0);
 }
 
 // Accumulate mode needs rows * (sum of N) fp32 inside the fixed 16 MiB region; larger outputs use ordered mode.
