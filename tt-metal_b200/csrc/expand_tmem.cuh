@@ -1,10 +1,9 @@
-// Expansion of packed bfloat8_b / bfloat4_b tiles into tensor memory as the bf16 A operand of tcgen05.mma, shared by the kernels
-// that multiply block-float weights from there (matmul_decode_tmem.cu, matmul_prefill.cu).
+// Expansion of packed bfloat8_b / bfloat4_b tiles into tensor memory as the bf16 A operand of tcgen05.mma, for matmul_rows.cu.
+// (matmul_decode_tmem.cu has an expansion of its own, for activations that tensor maps deliver in order.)
 //
 // A warp expands one 32x32 packed tile into the 32 TMEM lanes of its quadrant (lane = weight column) and 16 TMEM columns (two
-// K values each). What bounds it, from microbenchmarks per tile and scheduler: tcgen05.st 35 clocks (two 16x256b.x2; four .x1
-// took 54), the transposing loads 16 (bfloat4_b) or 32, the scale shuffles 20 - all of them through the same memory pipe - next
-// to 64 clocks of byte permutes and masks and 32 of multiplies.
+// K values each): two 16x256b.x2 stores, one (bfloat4_b) or two transposing loads and the scale shuffles, all of them through
+// the same memory pipe, next to byte permutes, masks and multiplies.
 #pragma once
 #include "epilogue.cuh"
 #include "sm100_ptx.cuh"
@@ -54,21 +53,19 @@ __device__ __forceinline__ uint32_t expand_ld_offset8(int lane) { return 64u + (
 // (sigma < 8) or lower face, with sigma chosen such that the four rows a lane receives (4q .. 4q+3, q = lane % 4) are K rows
 // 4q..4q+3 of the upper and 4(q^2)..4(q^2)+3 of the lower face. (The same K rows of both faces would put the eight addresses of
 // a phase on 64 bytes of banks twice.) K 16..31 of a block therefore stand in tensor memory with their halves of eight exchanged,
-// and the activations' copies exchange theirs (expand_b_swap). Without SWAP, for activations that tensor maps deliver in
-// order: rows 4q..4q+3 of both.
-template <bool SWAP>
+// and the activations' copies exchange theirs (expand_b_swap).
 __device__ __forceinline__ uint32_t expand_ld_offset4(int lane) {
     const int r16 = lane & 15;
     const int pair = (r16 >> 2) * 2 + (r16 & 1);   // rows 4q, 4q+1: pairs 2q, 2q+1 above; rows 4q+2, 4q+3: pairs 2(q^2), 2(q^2)+1 below
-    const uint32_t row = ((r16 >> 1) & 1) ? 256u + (uint32_t)(SWAP ? pair ^ 4 : pair) * 16u : (uint32_t)pair * 16u;
+    const uint32_t row = ((r16 >> 1) & 1) ? 256u + (uint32_t)(pair ^ 4) * 16u : (uint32_t)pair * 16u;
     return 64u + (uint32_t)(lane >> 4) * 128u + row;
 }
 // What to exclusive-or into the shared-memory address of a 16-byte chunk of the activation (operand B) whose K lies in the
 // second half of a K block.
 template <int FMT>
 constexpr uint32_t expand_b_swap = FMT == TTB_BFLOAT4_B ? 16u : 0u;
-template <int FMT, bool SWAP>
-__device__ __forceinline__ uint32_t expand_ld_offset(int lane) { return FMT == TTB_BFLOAT8_B ? expand_ld_offset8(lane) : expand_ld_offset4<SWAP>(lane); }
+template <int FMT>
+__device__ __forceinline__ uint32_t expand_ld_offset(int lane) { return FMT == TTB_BFLOAT8_B ? expand_ld_offset8(lane) : expand_ld_offset4(lane); }
 // Which of its quadrant's 32 weight columns a TMEM lane holds. bfloat8_b: the lane's own. bfloat4_b: a code byte carries two
 // neighbouring columns, and the transposing load hands the even one to lanes 0..7 and the odd one to lanes 8..15 of every
 // 16-lane half.
@@ -95,8 +92,8 @@ struct TileCodes {
 };
 
 // The lane whose scale pair belongs to this lane's first two K rows of face 2 * kh + nh (the next lane has the other two).
-template <int FMT, bool SWAP>
-__device__ __forceinline__ int expand_scale_lane(int nh, int kh, int sh0) { return 8 * (2 * kh + nh) + (SWAP && FMT == TTB_BFLOAT4_B && kh ? sh0 ^ 4 : sh0); }
+template <int FMT>
+__device__ __forceinline__ int expand_scale_lane(int nh, int kh, int sh0) { return 8 * (2 * kh + nh) + (FMT == TTB_BFLOAT4_B && kh ? sh0 ^ 4 : sh0); }
 
 // Column half `nh` (16 TMEM lanes) and K half `kh` of a tile: four registers of products.
 template <int FMT>
@@ -123,7 +120,7 @@ __device__ __forceinline__ void expand_quarter(const TileCodes<FMT> &c, int nh, 
 // One packed tile (shared address `tile`) -> the 32 TMEM lanes of this warp's quadrant, 16 columns at a_col. `sh0`: 2 * (lane % 4),
 // within a face's 8 scale pairs those of this lane's K rows.
 // BIG: some exponent of the tile exceeds 127 (a row maximum of 2 or more), whose power of two needs a second factor.
-template <int FMT, bool SWAP, bool BIG>
+template <int FMT, bool BIG>
 __device__ __forceinline__ void expand_tile(uint32_t tile, uint32_t a_col, uint32_t ld_off, uint32_t eh, int sh0) {
     const uint32_t my_scale = expand_scale(eh);
     const uint32_t my_t = BIG ? (__vmaxu2(__vminu2(eh, 0x00fe00feu), 0x007f007fu) << 7) : 0u;
@@ -134,7 +131,7 @@ __device__ __forceinline__ void expand_tile(uint32_t tile, uint32_t a_col, uint3
         uint32_t o[8];
 #pragma unroll
         for (int kh = 0; kh < 2; ++kh) {
-            const int f = expand_scale_lane<FMT, SWAP>(nh, kh, sh0);
+            const int f = expand_scale_lane<FMT>(nh, kh, sh0);
             expand_quarter<FMT>(c, nh, kh, __shfl_sync(0xffffffffu, my_scale, f), __shfl_sync(0xffffffffu, my_scale, f + 1), o + 4 * kh);
             if (BIG) {
                 const uint32_t t01 = __shfl_sync(0xffffffffu, my_t, f), t23 = __shfl_sync(0xffffffffu, my_t, f + 1);
@@ -146,14 +143,14 @@ __device__ __forceinline__ void expand_tile(uint32_t tile, uint32_t a_col, uint3
         tmem_st_16x256b_x2(a_col + ((uint32_t)(nh * 16) << 16), o);
     }
 }
-template <int FMT, bool SWAP>
+template <int FMT>
 __device__ __noinline__ void expand_tile_big(uint32_t tile, uint32_t a_col, uint32_t ld_off, uint32_t eh, int sh0) {
-    expand_tile<FMT, SWAP, true>(tile, a_col, ld_off, eh, sh0);
+    expand_tile<FMT, true>(tile, a_col, ld_off, eh, sh0);
 }
 
 // Two tiles at once (the common case: no exponent above 127): the transposing loads of both go out first and the faces
 // are expanded alternately, so that one tile's shuffles and stores wait behind the other's arithmetic.
-template <int FMT, bool SWAP>
+template <int FMT>
 __device__ __forceinline__ void expand_pair(uint32_t tile0, uint32_t tile1, uint32_t a_col0, uint32_t a_col1, uint32_t ld_off, uint32_t eh0, uint32_t eh1,
                                             int sh0) {
     TileCodes<FMT> c, d;
@@ -165,7 +162,7 @@ __device__ __forceinline__ void expand_pair(uint32_t tile0, uint32_t tile1, uint
         uint32_t o[8], w[8];
 #pragma unroll
         for (int kh = 0; kh < 2; ++kh) {
-            const int f = expand_scale_lane<FMT, SWAP>(nh, kh, sh0);
+            const int f = expand_scale_lane<FMT>(nh, kh, sh0);
             const uint32_t p01 = __shfl_sync(0xffffffffu, scale0, f), p23 = __shfl_sync(0xffffffffu, scale0, f + 1);
             const uint32_t q01 = __shfl_sync(0xffffffffu, scale1, f), q23 = __shfl_sync(0xffffffffu, scale1, f + 1);
             expand_quarter<FMT>(c, nh, kh, p01, p23, o + 4 * kh);
@@ -177,19 +174,19 @@ __device__ __forceinline__ void expand_pair(uint32_t tile0, uint32_t tile1, uint
 }
 
 // `count` (1 or 2) consecutive tiles `stride` bytes apart.
-template <int FMT, bool SWAP>
+template <int FMT>
 __device__ __forceinline__ void expand_tiles(uint32_t tile, uint32_t stride, uint32_t a_col, uint32_t a_stride, int count, uint32_t ld_off, int sh0, int lane) {
     const uint32_t eh0 = expand_exponents(tile, lane), eh1 = count > 1 ? expand_exponents(tile + stride, lane) : 0u;
     if (count > 1 && !__any_sync(0xffffffffu, ((eh0 | eh1) & 0x00800080u) != 0u)) {
-        expand_pair<FMT, SWAP>(tile, tile + stride, a_col, a_col + a_stride, ld_off, eh0, eh1, sh0);
+        expand_pair<FMT>(tile, tile + stride, a_col, a_col + a_stride, ld_off, eh0, eh1, sh0);
     } else {
         // a lone last tile, or an exponent above 127 somewhere (a row maximum of 2 or more): one tile at a time
         for (int t = 0; t < count; ++t) {
             const uint32_t e = t ? eh1 : eh0;
             if (__any_sync(0xffffffffu, (e & 0x00800080u) != 0u))
-                expand_tile_big<FMT, SWAP>(tile + t * stride, a_col + t * a_stride, ld_off, e, sh0);
+                expand_tile_big<FMT>(tile + t * stride, a_col + t * a_stride, ld_off, e, sh0);
             else
-                expand_tile<FMT, SWAP, false>(tile + t * stride, a_col + t * a_stride, ld_off, e, sh0);
+                expand_tile<FMT, false>(tile + t * stride, a_col + t * a_stride, ld_off, e, sh0);
         }
     }
 }

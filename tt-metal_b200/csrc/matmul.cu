@@ -25,7 +25,7 @@ int64_t prefill_workspace_bytes(int64_t rows, int64_t K);
 int32_t launch_matmul_prefill(const void *a, const void *w, int w_dtype, const void *bias, void *out, int out_dtype, int64_t rows,
                               int64_t K, int64_t N, int act, int flags, void *workspace, int64_t workspace_bytes, int *status,
                               cudaStream_t stream);
-int32_t launch_matmul_rows(const void *a, int count, const void *const *w, int w_dtype, const void *const *bias, void *const *out, int out_dtype, int64_t rows,
+int32_t launch_matmul_rows(const void *a, int count, const void *const *w, int w_dtype, const void *const *bias, void *const *out, int64_t rows,
                            int64_t K, const int64_t *N, int act, int flags, int *status, cudaStream_t stream);
 
 namespace {
@@ -213,7 +213,7 @@ int32_t ttb_matmul(const void *a, int32_t a_dtype, const void *w, int32_t w_dtyp
     int *status = nullptr;
     if (int32_t rc = status_word_address(&status)) return rc;
     if (kernel == TTB_KERNEL_BF16) return launch_matmul_bf16(a, w, bias, out, out_dtype, 1, rows, K, N, act, flags, status, s);
-    if (kernel == TTB_KERNEL_ROWS) return launch_matmul_rows(a, 1, &w, w_dtype, &bias, &out, out_dtype, rows, K, &N, act, flags, status, s);
+    if (kernel == TTB_KERNEL_ROWS) return launch_matmul_rows(a, 1, &w, w_dtype, &bias, &out, rows, K, &N, act, flags, status, s);
     RowChunk chunks[kMaxRowChunks];
     const int n = plan_rows(w_dtype, rows, K, N, chunks);
     const int64_t out_elem = out_dtype == TTB_FLOAT32 ? 4 : 2;

@@ -67,21 +67,6 @@ struct Args {
     long long wait_limit;   // of every barrier wait, in SM clocks
 };
 
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t local_addr, uint32_t rank) {
-    uint32_t addr;
-    float4 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local_addr), "r"(rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
-}
 // 32 bytes, in one store where the tensor allows it (the entry points ask for 16-byte alignment): a bfloat16 face row, so
 // that a warp's store covers whole 512-byte faces.
 __device__ __forceinline__ void store_32b(void *dst, const uint32_t (&v)[8], bool aligned32) {
@@ -127,7 +112,7 @@ __device__ __forceinline__ void finish_half(const Args &p, int64_t batch, int64_
     for (int q = 0; q < BN / 2; q += 16)
         if (n0 + q < p.N) {
             finish16<ACT>(p, batch, row, n0 + q, sum + q);
-            asm volatile("" ::: "memory");   // (keeps the compiler from fetching all groups' bias values at once, which spills)
+            asm volatile("" ::: "memory");   // (keeps the compiler from fetching all groups' bias values at once, which spills more)
         }
 }
 

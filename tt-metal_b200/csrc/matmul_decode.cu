@@ -24,7 +24,7 @@ static constexpr int64_t kCounterBytes = 65536;
 static constexpr int64_t kAccumBytes = 16 << 20;
 
 int32_t launch_decode_tmem(const DecodeArgs *stages, int n, int fmt, int nb, int *sync, bool overlap, cudaStream_t stream);
-int32_t launch_matmul_rows(const void *a, int count, const void *const *w, int w_dtype, const void *const *bias, void *const *out, int out_dtype, int64_t rows,
+int32_t launch_matmul_rows(const void *a, int count, const void *const *w, int w_dtype, const void *const *bias, void *const *out, int64_t rows,
                            int64_t K, const int64_t *N, int act, int flags, int *status, cudaStream_t stream);
 // The tail of the counter region belongs to the launch as a whole (matmul_decode_tmem.cu: blocks that have finished, tiles
 // each stage has stored); the per-tile counters stay below it.
@@ -576,7 +576,7 @@ extern "C" int32_t ttb_matmul_multi(const void *a, int32_t a_dtype, int32_t coun
         !decode_is_faster(rows, K, tiles, any_ragged(count, N))) {
         int *status = nullptr;
         if (int32_t rc = status_word_address(&status)) return rc;
-        return launch_matmul_rows(a, count, w, w_dtype, bias, out, out_dtype, rows, K, N, act, flags, status, (cudaStream_t)stream);
+        return launch_matmul_rows(a, count, w, w_dtype, bias, out, rows, K, N, act, flags, status, (cudaStream_t)stream);
     }
     return launch_matmul_decode_multi(a, count, w, w_dtype, bias, out, out_dtype, rows, K, N, act,
                                       flags & (TTB_MM_A_ROW_MAJOR | TTB_MM_OUT_ROW_MAJOR | TTB_MM_DETERMINISTIC | TTB_MM_WEIGHTS_RESIDENT | TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_GATED),

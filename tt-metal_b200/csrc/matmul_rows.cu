@@ -79,26 +79,10 @@ struct alignas(64) Args {
     int chunks, chunk_rows; // row chunks and rows of each (the last may have fewer)
     int tile0, tiles;       // this launch's tiles: tile0 .. tile0 + tiles - 1; row chunks vary fastest
     int split;              // blocks (= cluster size) that share a tile's K range
-    int act, out_dtype, a_row_major, out_row_major;
+    int act, a_row_major, out_row_major;
     int *status;
     long long wait_limit;   // of every barrier wait, in SM clocks
 };
-
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t local_addr, uint32_t rank) {
-    uint32_t addr;
-    float4 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local_addr), "r"(rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
-}
 
 // Four neighbouring columns n .. n + 3 of one row: bias, activation, store.
 template <int ACT>
@@ -106,12 +90,9 @@ __device__ __forceinline__ void finish4(const Args &p, int w, int64_t row, int64
     v.x = apply_activation_t<ACT>(v.x + b.x); v.y = apply_activation_t<ACT>(v.y + b.y);
     v.z = apply_activation_t<ACT>(v.z + b.z); v.w = apply_activation_t<ACT>(v.w + b.w);
     const int64_t off = p.out_row_major ? row * p.N[w] + n : tiled_offset(row, n, p.N[w] >> 5);
-    if (p.out_dtype == TTB_FLOAT32)
-        *reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.out[w]) + off) = v;
-    else
-        *reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(p.out[w]) + off) =
-            make_uint2((uint32_t)f32_to_bf16_bits(v.x) | ((uint32_t)f32_to_bf16_bits(v.y) << 16),
-                       (uint32_t)f32_to_bf16_bits(v.z) | ((uint32_t)f32_to_bf16_bits(v.w) << 16));
+    *reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(p.out[w]) + off) =
+        make_uint2((uint32_t)f32_to_bf16_bits(v.x) | ((uint32_t)f32_to_bf16_bits(v.y) << 16),
+                   (uint32_t)f32_to_bf16_bits(v.z) | ((uint32_t)f32_to_bf16_bits(v.w) << 16));
 }
 __device__ __forceinline__ float4 bias4(const Args &p, int w, int64_t n) {
     if (!p.bias[w] || n >= p.N[w]) return make_float4(0.f, 0.f, 0.f, 0.f);
@@ -197,7 +178,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
     if (warp < kExpandWarps) {
         // ---------------- expand warps: packed codes -> bf16 in tensor memory ----------------
         const int team = warp >> 2, quad = warp & 3;
-        const uint32_t ld_off = expand_ld_offset<FMT, true>(lane);
+        const uint32_t ld_off = expand_ld_offset<FMT>(lane);
         const int sh0 = 2 * (lane & 3);
         const uint32_t pk_quad = sbase + L::pk + quad * L::kTile;
         const uint32_t a_quad = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)kACol0;
@@ -215,7 +196,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
                 if (count > 0) {
                     const int j = team * (kGroup / kTeams);
                     tc_fence_after_sync();
-                    expand_tiles<FMT, true>(pk_quad + (uint32_t)((ps * kGroup + j) * L::kPStageBytes), L::kPStageBytes,
+                    expand_tiles<FMT>(pk_quad + (uint32_t)((ps * kGroup + j) * L::kPStageBytes), L::kPStageBytes,
                                             a_quad + (uint32_t)((gs * kGroup + j) * kAColsPerStage), kAColsPerStage, count, ld_off, sh0, lane);
                     tmem_st_wait();
                     tc_fence_before_sync();
@@ -514,13 +495,13 @@ int32_t launch_fmt(Args &p, bool overlap, cudaStream_t stream) {
 }
 }  // namespace
 
-// `count` matmuls that share the activation, in one or two launches, whatever the row and column counts.
-int32_t launch_matmul_rows(const void *a, int count, const void *const *w, int w_dtype, const void *const *bias, void *const *out, int out_dtype, int64_t rows,
+// `count` matmuls with bfloat16 results that share the activation, in one or two launches, whatever the row and column counts.
+int32_t launch_matmul_rows(const void *a, int count, const void *const *w, int w_dtype, const void *const *bias, void *const *out, int64_t rows,
                            int64_t K, const int64_t *N, int act, int flags, int *status, cudaStream_t stream) {
     Args p = {};
     p.a = (const uint16_t *)a;
     p.rows = rows; p.K = K; p.Kt = (int)(K / BK);
-    p.act = act; p.out_dtype = out_dtype;
+    p.act = act;
     p.a_row_major = (flags & TTB_MM_A_ROW_MAJOR) != 0;
     p.out_row_major = (flags & TTB_MM_OUT_ROW_MAJOR) != 0;
     p.status = status;
