@@ -93,6 +93,7 @@ int32_t ttb_free(void *dev_ptr);
 int32_t ttb_mem_info(int64_t *free_bytes, int64_t *total_bytes);
 int32_t ttb_host_alloc(void **host_ptr, size_t bytes); /* pinned host memory */
 int32_t ttb_host_free(void *host_ptr);
+/* Copies from and to pageable host memory may be complete when these return, as with the CUDA runtime; from 4 MiB on they are. */
 int32_t ttb_memcpy_h2d(void *dst_dev, const void *src_host, size_t bytes, void *stream);
 int32_t ttb_memcpy_d2h(void *dst_host, const void *src_dev, size_t bytes, void *stream);
 int32_t ttb_memcpy_d2d(void *dst_dev, const void *src_dev, size_t bytes, void *stream);
@@ -164,8 +165,8 @@ int32_t ttb_unpack_bfp(const void *src_dev, int32_t fmt, void *dst_dev, int32_t 
  *   bias: NULL, or TTB_BFLOAT16 tiled [32, N] whose first row is used (the reference's
  *         [1,1,32,N] bias tile row, tt_eager/tt_dnn/op_library/bmm/bmm_op.cpp:859-863).
  *   out:  TTB_BFLOAT16 or TTB_FLOAT32, tiled (or row-major with TTB_MM_OUT_ROW_MAJOR).
- * Block-float weights are expanded to bf16 in shared memory (exact) and multiplied on the tcgen05
- * tensor cores, bf16 weights go there as they are; shapes outside the tensor-core kernels' tiling use a CUDA-core kernel
+ * Block-float weights are expanded to bf16 on the chip (exact) and multiplied on the tcgen05
+ * tensor cores, bf16 weights go there as they are; what the tensor-core kernels do not take uses a CUDA-core kernel
  * with the same arithmetic. Stands in for tt::operations::primary::matmul and the multi-core-reuse program
  * factories (bmm_op.hpp:284-346, bmm_op.cpp:828-1303, and the multi_core_reuse program factories
  * beside them). `workspace` is device scratch of at least ttb_matmul_workspace_bytes() bytes (may be NULL when
@@ -174,7 +175,8 @@ int32_t ttb_unpack_bfp(const void *src_dev, int32_t fmt, void *dst_dev, int32_t 
  * memset on `stream` unless TTB_MM_WORKSPACE_ZEROED is given. */
 int64_t ttb_matmul_workspace_bytes(int32_t w_dtype, int64_t batch, int64_t M, int64_t K, int64_t N, int32_t flags);
 /* Which kernel computes a call of ttb_matmul (no GPU needed; the answer without one is a B200's): one of these, or a negative
- * TTB_E_* for sizes, types or flags that ttb_matmul refuses. */
+ * TTB_E_* for sizes, types or flags that ttb_matmul refuses. (With the workspace that ttb_matmul_workspace_bytes asks for; without it
+ * bfloat16 results of 96 rows and more run as TTB_KERNEL_ROWS.) */
 #define TTB_KERNEL_GENERIC 0 /* CUDA cores, any shape */
 #define TTB_KERNEL_RANGES 1  /* decode and prefill kernels over row ranges: ttb_matmul_plan has them */
 #define TTB_KERNEL_ROWS 2    /* block-float weights, bfloat16 results, any row and column count: csrc/matmul_rows.cu */
@@ -196,7 +198,8 @@ int32_t ttb_matmul(const void *a_dev, int32_t a_dtype, const void *w_dev, int32_
  * `a` bfloat16, `w` bfloat8_b / bfloat4_b / bfloat16 (one packed [K, N] matrix after the other), fp32 accumulation, bfloat16 or
  * float32 output. Stands in for tt::tt_metal::bmm and the batched form of tt::operations::primary::matmul
  * (tt_eager/tt_dnn/op_library/bmm/bmm_op.hpp:388-456, bmm_op.cpp:518-626; attention's Q K^T and P V products,
- * tests/tt_eager/python_api_testing/unit_testing/misc/test_matmul.py:204-320). Runs on the CUDA cores. */
+ * tests/tt_eager/python_api_testing/unit_testing/misc/test_matmul.py:204-320). bfloat16 `w` runs on the tensor cores (but for short
+ * sums of small or fp32 results), block-float `w` on the CUDA cores. */
 int32_t ttb_bmm(const void *a_dev, int32_t a_dtype, const void *w_dev, int32_t w_dtype, void *out_dev, int32_t out_dtype, int64_t batch,
                 int64_t M, int64_t K, int64_t N, void *stream);
 

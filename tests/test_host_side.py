@@ -222,3 +222,21 @@ def test_small_bfloat16_products_take_the_kernel_that_measured_faster(fake, batc
     assert len(log) == 1 and ("matmul_bf16_kernel" in log[0]) == tensor_cores, log
     if batch == 1:
         assert kernel(fake, M, K, N, cabi.BFLOAT16) == (cabi.KERNEL_BF16 if tensor_cores else cabi.KERNEL_GENERIC)
+
+
+@pytest.mark.parametrize("M,K,N", [(96, 28672, 256), (256, 20480, 128), (1024, 8192, 9472), (512, 512, 18944)])
+@pytest.mark.parametrize("workspace,nbytes", [(None, 0), (1 << 40, 16), ((1 << 40) + 16, 1 << 40)])
+def test_calls_without_scratch_get_the_kernel_that_needs_none(fake, M, K, N, workspace, nbytes):
+    """Shapes that go to the decode or prefill kernel with the workspace they ask for: with none, too little or a misaligned one they
+    are served all the same; under MM_DETERMINISTIC, which only those kernels serve, they are refused."""
+    assert kernel(fake, M, K, N) == cabi.KERNEL_RANGES and fake.matmul_workspace_bytes(cabi.BFLOAT8_B, 1, M, K, N, 0) > 0
+    run = lambda flags: fake.cdll.ttb_matmul(4096, cabi.BFLOAT16, 8192, cabi.BFLOAT8_B, None, 1 << 20, cabi.BFLOAT16, 1, M, K, N, 0, flags, workspace, nbytes, None)   # noqa: E731
+    fake.cdll.fake_log()
+    assert run(0) == 0
+    log = fake.cdll.fake_log().decode().split()
+    assert log and all("matmul_rows" in k for k in log), log
+    assert run(cabi.MM_DETERMINISTIC) in (-1, -4) and not fake.cdll.fake_log()
+    if M <= 256:
+        assert fake.cdll.ttb_matmul_multi(4096, cabi.BFLOAT16, 1, (ctypes.c_void_p * 1)(1 << 34), cabi.BFLOAT8_B, None, (ctypes.c_void_p * 1)(1 << 35), cabi.BFLOAT16, 1,
+                                          M, K, (ctypes.c_int64 * 1)(N), 0, 0, workspace, nbytes, None, None, None) == 0
+        assert "matmul_rows" in fake.cdll.fake_log().decode()

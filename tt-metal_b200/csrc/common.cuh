@@ -48,6 +48,11 @@ class Once {
     }
 };
 
+// Whether a caller's scratch is what a launch of the kernels that need it asks for.
+inline bool workspace_serves(const void *workspace, int64_t bytes, int64_t need) {
+    return need == 0 || (workspace && bytes >= need && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0);
+}
+
 constexpr int kTile = 32;
 constexpr int kTileElems = 1024;
 constexpr int kBfp8TileBytes = 1088;

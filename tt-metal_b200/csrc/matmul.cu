@@ -104,9 +104,12 @@ bool prefill_is_faster(int w_dtype, int64_t rows, int64_t K, int64_t N) {
 //    27.1, 64 x 4096 x 1024 14.2 / 8.0, 64 x 8192 x 9472 (74 tiles) 34.1 / 28.1, but 64 x 8192 x 9600 (75 tiles) 34.0 / 46.0; up to a K
 //    at which that is so for any column count (64 x 20480 x 512 15.8 / 17.0);
 //  * where the prefill kernel applies, except for the shapes that it keeps.
-bool rows_kernel_takes(int w_dtype, int out_dtype, int64_t rows, int64_t K, int64_t N, int flags) {
+bool rows_kernel_can(int w_dtype, int out_dtype, int flags) {
     // (under TTB_MM_DETERMINISTIC a call gives the bytes of the same stage of a sequence, which the decode kernel computes)
-    if (w_dtype == TTB_BFLOAT16 || out_dtype != TTB_BFLOAT16 || (flags & (TTB_MM_FORCE_GENERIC | TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_DETERMINISTIC))) return false;
+    return w_dtype != TTB_BFLOAT16 && out_dtype == TTB_BFLOAT16 && !(flags & (TTB_MM_FORCE_GENERIC | TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_DETERMINISTIC));
+}
+bool rows_kernel_takes(int w_dtype, int out_dtype, int64_t rows, int64_t K, int64_t N, int flags) {
+    if (!rows_kernel_can(w_dtype, out_dtype, flags)) return false;
     if (rows == 64) return (N + 127) / 128 * 2 <= stream_blocks() && K <= 8192;
     if (rows < 96) return false;
     if (rows <= 256) return !(decode_supported(w_dtype, rows, K, N) && decode_is_faster(rows, K, (N + 127) / 128, N % 128 != 0));
@@ -208,7 +211,11 @@ int32_t ttb_matmul(const void *a, int32_t a_dtype, const void *w, int32_t w_dtyp
     if (int32_t rc = validate(a, a_dtype, w, w_dtype, out, out_dtype, batch, M, K, N, act)) return rc;
     const int64_t rows = batch * M;  // tiled [batch, M, K] with M % 32 == 0 is the same buffer as tiled [batch*M, K]
     auto s = (cudaStream_t)stream;
-    const int kernel = kernel_of(w_dtype, out_dtype, rows, K, N, flags);
+    int kernel = kernel_of(w_dtype, out_dtype, rows, K, N, flags);
+    // (a call that brings no scratch still gets the kernel that needs none)
+    if (kernel == TTB_KERNEL_RANGES && rows >= 96 && rows_kernel_can(w_dtype, out_dtype, flags) &&
+        !workspace_serves(workspace, workspace_bytes, ttb_matmul_workspace_bytes(w_dtype, batch, M, K, N, flags)))
+        kernel = TTB_KERNEL_ROWS;
     if (kernel == TTB_KERNEL_GENERIC) return launch_matmul_generic(a, w, w_dtype, bias, out, out_dtype, rows, K, N, act, flags, s);
     int *status = nullptr;
     if (int32_t rc = status_word_address(&status)) return rc;

@@ -1,5 +1,5 @@
 // Host side of the decode (small row count) matmuls: planning of the streamed decomposition, workspace layout, dispatch
-// to the kernels (matmul_decode_stream.cu; matmul_decode_tmem.cu for 128-row blocks of bfloat8_b), the allocation-free
+// to the kernels (matmul_decode_tmem.cu; matmul_decode_stream.cu on request), the allocation-free
 // entry point, the entry point whose epilogue is the all-gather, and the device status word of the bounded waits.
 #include <type_traits>
 
@@ -573,7 +573,8 @@ extern "C" int32_t ttb_matmul_multi(const void *a, int32_t a_dtype, int32_t coun
     int64_t tiles = 0;
     for (int j = 0; j < count; ++j) tiles += tiles128(N[j]);
     if (rows >= 96 && out_dtype == TTB_BFLOAT16 && !gather && !wait && !(flags & (TTB_MM_DECODE_SMEM_OPERAND | TTB_MM_GATED | TTB_MM_DETERMINISTIC)) &&
-        !decode_is_faster(rows, K, tiles, any_ragged(count, N))) {
+        !(decode_is_faster(rows, K, tiles, any_ragged(count, N)) &&
+          workspace_serves(workspace, workspace_bytes, decode_workspace_bytes_multi(rows, K, count, N, false)))) {   // (no scratch: the kernel that needs none)
         int *status = nullptr;
         if (int32_t rc = status_word_address(&status)) return rc;
         return launch_matmul_rows(a, count, w, w_dtype, bias, out, rows, K, N, act, flags, status, (cudaStream_t)stream);
