@@ -218,9 +218,11 @@ int32_t ttb_matmul(const void *a, int32_t a_dtype, const void *w, int32_t w_dtyp
         kernel = TTB_KERNEL_ROWS;
     if (kernel == TTB_KERNEL_GENERIC) return launch_matmul_generic(a, w, w_dtype, bias, out, out_dtype, rows, K, N, act, flags, s);
     int *status = nullptr;
-    if (int32_t rc = status_word_address(&status)) return rc;
-    if (kernel == TTB_KERNEL_BF16) return launch_matmul_bf16(a, w, bias, out, out_dtype, 1, rows, K, N, act, flags, status, s);
-    if (kernel == TTB_KERNEL_ROWS) return launch_matmul_rows(a, 1, &w, w_dtype, &bias, &out, rows, K, &N, act, flags, status, s);
+    if (kernel != TTB_KERNEL_RANGES) {
+        if (int32_t rc = status_word_address(&status)) return rc;
+        if (kernel == TTB_KERNEL_BF16) return launch_matmul_bf16(a, w, bias, out, out_dtype, 1, rows, K, N, act, flags, status, s);
+        return launch_matmul_rows(a, 1, &w, w_dtype, &bias, &out, rows, K, &N, act, flags, status, s);
+    }
     RowChunk chunks[kMaxRowChunks];
     const int n = plan_rows(w_dtype, rows, K, N, chunks);
     const int64_t out_elem = out_dtype == TTB_FLOAT32 ? 4 : 2;
@@ -229,6 +231,7 @@ int32_t ttb_matmul(const void *a, int32_t a_dtype, const void *w, int32_t w_dtyp
         void *oi = static_cast<uint8_t *>(out) + chunks[i].row0 * N * out_elem;
         int32_t rc;
         if (chunks[i].prefill) {
+            if ((rc = status_word_address(&status))) return rc;
             rc = launch_matmul_prefill(ai, w, w_dtype, bias, oi, out_dtype, chunks[i].rows, K, N, act, flags, workspace, workspace_bytes, status, s);
         } else {
             rc = launch_matmul_decode(ai, w, w_dtype, bias, oi, out_dtype, chunks[i].rows, K, N, act, flags, workspace, workspace_bytes,
