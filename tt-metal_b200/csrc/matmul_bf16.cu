@@ -30,7 +30,7 @@
 #include "sm100_ptx.cuh"
 
 namespace ttb {
-long long barrier_limit_cycles();
+unsigned barrier_limit_kcycles();
 namespace {
 
 using namespace ptx;
@@ -63,9 +63,11 @@ struct Args {
     int nstages;                           // stages of the whole K range
     int chunk;                             // stages per accumulator
     int act, out_dtype, a_row_major, out_row_major, out_aligned32;
+    unsigned wait_limit;   // of every barrier wait, in 1024 SM clocks
     int *status;
-    long long wait_limit;   // of every barrier wait, in SM clocks
 };
+
+__device__ __forceinline__ long long wait_clocks(const Args &p) { return (long long)p.wait_limit << 10; }
 
 // 32 bytes, in one store where the tensor allows it (the entry points ask for 16-byte alignment): a bfloat16 face row, so
 // that a warp's store covers whole 512-byte faces.
@@ -181,7 +183,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_bf16_kernel(const __grid_c
             locate(tile, b, m, n);
             const uint16_t *const ab = p.a + b * p.a_bstride, *const wb = p.w + b * p.w_bstride;
             for (int st = st0; st < st1; ++st) {
-                if (!__all_sync(0xffffffffu, mbar_wait(empty(s), ph ^ 1, abort_flag, p.status, 41, p.wait_limit))) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(empty(s), ph ^ 1, abort_flag, p.status, 41, wait_clocks(p)))) { ok = false; break; }
                 const uint32_t dst = sbase + s * kStageBytes;
                 // eight tiles per operand: this warp takes tile row (column) pw of each of the stage's two K tiles
 #pragma unroll
@@ -229,10 +231,10 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_bf16_kernel(const __grid_c
         for (int tile = first_tile; ok && tile < p.tiles; tile += tile_step) {
             for (int st = st0; ok && st < st1; st += p.chunk, ++c) {
                 const int buf = c & 1;
-                if (!__all_sync(0xffffffffu, mbar_wait(acc_empty(buf), (uint32_t)(((c >> 1) & 1) ^ 1), abort_flag, p.status, 42, p.wait_limit))) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(acc_empty(buf), (uint32_t)(((c >> 1) & 1) ^ 1), abort_flag, p.status, 42, wait_clocks(p)))) { ok = false; break; }
                 const int end = min(st1, st + p.chunk);
                 for (int i = st; i < end; ++i) {
-                    if (!__all_sync(0xffffffffu, mbar_wait(full(s), ph, abort_flag, p.status, 43, p.wait_limit))) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(full(s), ph, abort_flag, p.status, 43, wait_clocks(p)))) { ok = false; break; }
                     // The copies are generic-proxy writes; ordering them here, before the MMAs read them, and not in the producers
                     // keeps the producers' later copies flowing (a fence there waits for those too: 31 B per clock).
                     fence_proxy_async_smem();
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_bf16_kernel(const __grid_c
             for (int j = 0; j < BN / 2; ++j) sum[j] = 0.0f;
             for (int st = st0; st < st1; st += p.chunk, ++c) {
                 const int buf = c & 1;
-                if (!__all_sync(0xffffffffu, mbar_wait(acc_full(buf), (uint32_t)((c >> 1) & 1), abort_flag, p.status, 44, p.wait_limit))) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(acc_full(buf), (uint32_t)((c >> 1) & 1), abort_flag, p.status, 44, wait_clocks(p)))) { ok = false; break; }
                 tc_fence_after_sync();
 #pragma unroll
                 for (int q = 0; q < BN / 2; q += 32) {
@@ -359,7 +361,7 @@ int32_t launch_matmul_bf16(const void *a, const void *w, const void *bias, void 
     p.out_row_major = (flags & TTB_MM_OUT_ROW_MAJOR) != 0;
     p.out_aligned32 = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
     p.status = status;
-    p.wait_limit = barrier_limit_cycles();
+    p.wait_limit = barrier_limit_kcycles();
     const int64_t mt = (rows + BM - 1) / BM, nt = (N + BN - 1) / BN, tiles = mt * nt * batch;
     if (tiles > INT32_MAX / 8 || K / 32 > INT32_MAX || N / 32 > INT32_MAX) return fail(TTB_E_UNSUPPORTED, "ttb_matmul: too many output tiles");
     p.mt = (int)mt; p.nt = (int)nt; p.tiles = (int)tiles;

@@ -12,8 +12,11 @@ __device__ int g_status_word = 0;
 // Limit of the bounded device-side waits in SM clocks; 0 = each wait's built-in default. Read at launch time.
 static long long g_wait_limit_cycles = 0;
 long long wait_limit_cycles() { return g_wait_limit_cycles; }
-// ... of the pipeline barriers of a kernel that waits for no peers itself.
-long long barrier_limit_cycles() { return g_wait_limit_cycles > 0 ? 2 * g_wait_limit_cycles + 1000000LL : 2000000000LL; }
+// ... of the pipeline barriers of a kernel that waits for no peers itself, in units of 1024 clocks.
+unsigned barrier_limit_kcycles() {
+    const long long kc = g_wait_limit_cycles > 0 ? (g_wait_limit_cycles >> 9) + 978 : 1953125;   // 2 * limit + 1,000,000 clocks; 2,000,000,000
+    return kc < 0xffffffffLL ? (unsigned)kc : 0xffffffffu;
+}
 
 using namespace decode_smem;
 

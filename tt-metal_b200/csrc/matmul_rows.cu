@@ -28,7 +28,7 @@
 #include "expand_tmem.cuh"
 
 namespace ttb {
-long long barrier_limit_cycles();
+unsigned barrier_limit_kcycles();
 namespace {
 
 using namespace ptx;
@@ -80,9 +80,11 @@ struct alignas(64) Args {
     int tile0, tiles;       // this launch's tiles: tile0 .. tile0 + tiles - 1; row chunks vary fastest
     int split;              // blocks (= cluster size) that share a tile's K range
     int act, a_row_major, out_row_major;
+    unsigned wait_limit;   // of every barrier wait, in 1024 SM clocks
     int *status;
-    long long wait_limit;   // of every barrier wait, in SM clocks
 };
+
+__device__ __forceinline__ long long wait_clocks(const Args &p) { return (long long)p.wait_limit << 10; }
 
 // Four neighbouring columns n .. n + 3 of one row: bias, activation, store.
 template <int ACT>
@@ -116,6 +118,14 @@ __device__ __forceinline__ void finish_rows(const Args &p, int w, uint32_t slab,
         }
         finish4<ACT>(p, w, row_base + r, n, v, b);
     }
+}
+
+// A bounded wait whose barrier may depend on the previous kernel: that one's time is not to count. (What is free at once is free
+// without it; the wait for it returns at once ever after.)
+__device__ __forceinline__ bool mbar_wait_behind(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code, long long limit) {
+    if (mbar_try_wait(bar, parity)) return true;
+    grid_dep_wait();
+    return mbar_wait(bar, parity, abort_flag, status, code, limit);
 }
 
 template <int FMT, int BR>
@@ -182,13 +192,12 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
         const int sh0 = 2 * (lane & 3);
         const uint32_t pk_quad = sbase + L::pk + quad * L::kTile;
         const uint32_t a_quad = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)kACol0;
-        int gs = 0, ps = 0, ahead = kRing;   // groups that go before the first MMA
+        int gs = 0, ps = 0;
         uint32_t ph = 0, pph = 0;
         bool ok = true;
         for (int t = first; ok && t < p.tiles; t += step) {
             for (int kb = kb0; kb < kb1; kb += kGroup) {
-                if (ahead-- == 0) grid_dep_wait();   // the MMAs wait for the previous kernel: its time is not this barrier's
-                if (!__all_sync(0xffffffffu, mbar_wait(full_p(ps), pph, abort_flag, p.status, 51, p.wait_limit) && mbar_wait(empty(gs), ph ^ 1u, abort_flag, p.status, 52, p.wait_limit))) {
+                if (!__all_sync(0xffffffffu, mbar_wait(full_p(ps), pph, abort_flag, p.status, 51, wait_clocks(p)) && mbar_wait_behind(empty(gs), ph ^ 1u, abort_flag, p.status, 52, wait_clocks(p)))) {
                     ok = false;
                     break;
                 }
@@ -220,8 +229,8 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
             int w;
             const int nt = column_tile_of(t, w);
             for (int kb = kb0; kb < kb1; kb += kGroup) {
-                if (ahead-- == 0) grid_dep_wait();   // (as above: the expand warps have emptied kRing groups by then)
-                if (!__all_sync(0xffffffffu, mbar_wait(empty_p(s), ph ^ 1u, abort_flag, p.status, 53, p.wait_limit))) { ok = false; break; }
+                if (ahead-- == 0) grid_dep_wait();   // (the expand warps have emptied kRing groups by then; the next one follows an MMA)
+                if (!__all_sync(0xffffffffu, mbar_wait(empty_p(s), ph ^ 1u, abort_flag, p.status, 53, wait_clocks(p)))) { ok = false; break; }
                 if (leader) {
                     // (always a whole box: what lies beyond the weight reads as zeros, a surplus K block is not expanded)
                     mbar_arrive_expect_tx(full_p(s), kGroup * L::kPStageBytes);
@@ -252,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
                 down = 512; right = 256; next_k = 1024; next_row = (int64_t)kLoaderWarps * p.Kt * 1024;
             }
             for (int kb = kb0; kb < kb1; kb += kGroup) {
-                if (!__all_sync(0xffffffffu, mbar_wait(empty(s), ph ^ 1u, abort_flag, p.status, 54, p.wait_limit))) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(empty(s), ph ^ 1u, abort_flag, p.status, 54, wait_clocks(p)))) { ok = false; break; }
                 uint32_t d0 = sbase + L::x + s * kGroup * kXStageBytes + lw * 1024 + face_dst;
                 for (int j = 0; j < min(kGroup, kb1 - kb); ++j, src += next_k, d0 += kXStageBytes) {
                     const uint16_t *f = src;
@@ -281,11 +290,11 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
         uint32_t ph = 0;
         bool ok = true;
         for (int t = first; ok && t < p.tiles; t += step, ++n) {
-            if (!__all_sync(0xffffffffu, mbar_wait(acc_empty, (uint32_t)((n & 1) ^ 1), abort_flag, p.status, 55, p.wait_limit))) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(acc_empty, (uint32_t)((n & 1) ^ 1), abort_flag, p.status, 55, wait_clocks(p)))) { ok = false; break; }
             tc_fence_after_sync();
             const uint32_t idesc = instr_desc_bf16_f32(BN, 0, /*a_mn_major=*/false, /*b_mn_major=*/false) | ((uint32_t)(rows_of(chunk_of(t)) >> 3) << 17);
             for (int kb = kb0; kb < kb1; kb += kGroup) {
-                if (!__all_sync(0xffffffffu, mbar_wait(full(gs), ph, abort_flag, p.status, 56, p.wait_limit))) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_wait(full(gs), ph, abort_flag, p.status, 56, wait_clocks(p)))) { ok = false; break; }
                 fence_proxy_async_smem();   // the activations came through the generic proxy
                 tc_fence_after_sync();
                 const uint32_t a_col = tmem_base + (uint32_t)(kACol0 + gs * kGroup * kAColsPerStage);
@@ -321,7 +330,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_rows_kernel(const __grid_c
             int w;
             const int64_t row_base = (int64_t)chunk * p.chunk_rows, col0 = (int64_t)column_tile_of(t, w) * BN + lane * 4;
             // (the eight warps meet at named barriers below: they go on together or not at all)
-            int good = mbar_wait(acc_full, (uint32_t)(n & 1), abort_flag, p.status, 57, p.wait_limit) ? 1 : 0;
+            int good = mbar_wait(acc_full, (uint32_t)(n & 1), abort_flag, p.status, 57, wait_clocks(p)) ? 1 : 0;
             asm volatile(
                 "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %0, 0;\n\tbarrier.cta.red.and.pred q, 1, %1, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
                 : "+r"(good)
@@ -505,7 +514,7 @@ int32_t launch_matmul_rows(const void *a, int count, const void *const *w, int w
     p.a_row_major = (flags & TTB_MM_A_ROW_MAJOR) != 0;
     p.out_row_major = (flags & TTB_MM_OUT_ROW_MAJOR) != 0;
     p.status = status;
-    p.wait_limit = barrier_limit_cycles();
+    p.wait_limit = barrier_limit_kcycles();
     p.weights = count;
     int64_t tiles = 0;
     for (int j = 0; j < count; ++j) {
