@@ -82,9 +82,10 @@ __device__ __forceinline__ void store_32b(void *dst, const uint32_t (&v)[8], boo
     }
 }
 
-// 16 columns from n0 of one row: bias, activation, store.
+// 16 columns from n0 of one row: bias, activation, store. (Coordinates in 32 bits: 64 took the kernel from 4 bytes of register
+// spills to 148 and a 1024 x 1024 x 1024 launch from 9.3 us to 9.9.)
 template <int ACT>
-__device__ __forceinline__ void finish16(const Args &p, int64_t batch, int64_t row, int64_t n0, float *v) {
+__device__ __forceinline__ void finish16(const Args &p, int batch, int row, int n0, float *v) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         if (p.bias) v[j] += bias_at(p.bias, n0 + j);
@@ -109,12 +110,12 @@ __device__ __forceinline__ void finish16(const Args &p, int64_t batch, int64_t r
 
 // One thread's half row of a tile.
 template <int ACT>
-__device__ __forceinline__ void finish_half(const Args &p, int64_t batch, int64_t row, int64_t n0, float (&sum)[BN / 2]) {
+__device__ __forceinline__ void finish_half(const Args &p, int batch, int row, int n0, float (&sum)[BN / 2]) {
 #pragma unroll
     for (int q = 0; q < BN / 2; q += 16)
         if (n0 + q < p.N) {
             finish16<ACT>(p, batch, row, n0 + q, sum + q);
-            asm volatile("" ::: "memory");   // (keeps the compiler from fetching all groups' bias values at once, which spills more)
+            asm volatile("" ::: "memory");   // (keeps the compiler from fetching all groups' bias values at once, which spills)
         }
 }
 
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_bf16_kernel(const __grid_c
                 if (lane == 0) mbar_arrive(acc_empty(buf));
             }
             if (!ok) break;
-            const int64_t row = (int64_t)m * BM + quad * 32 + lane;
+            const int row = m * BM + quad * 32 + lane;
             const int col = n * BN + half * (BN / 2);
             if (p.split == 1) {
                 if (row < p.rows) TTB_DISPATCH_ACT(p.act, finish_half<ACT>(p, b, row, col, sum));
@@ -309,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_bf16_kernel(const __grid_c
             const int quad = warp & 3, half = warp >> 2;
             int b, m, n;
             locate(first_tile, b, m, n);
-            const int64_t row = (int64_t)m * BM + quad * 32 + lane;
+            const int row = m * BM + quad * 32 + lane;
             const int units = BN / 16 / p.split;   // columns in groups of 16
             if (row < p.rows)
                 for (int u = half; u < units; u += 2) {
@@ -363,7 +364,7 @@ int32_t launch_matmul_bf16(const void *a, const void *w, const void *bias, void 
     p.status = status;
     p.wait_limit = barrier_limit_kcycles();
     const int64_t mt = (rows + BM - 1) / BM, nt = (N + BN - 1) / BN, tiles = mt * nt * batch;
-    if (tiles > INT32_MAX / 8 || K / 32 > INT32_MAX || N / 32 > INT32_MAX) return fail(TTB_E_UNSUPPORTED, "ttb_matmul: too many output tiles");
+    if (tiles > INT32_MAX / 8 || K / 32 > INT32_MAX || rows > INT32_MAX - BM || N > INT32_MAX - BN) return fail(TTB_E_UNSUPPORTED, "ttb_matmul: too many output tiles");
     p.mt = (int)mt; p.nt = (int)nt; p.tiles = (int)tiles;
     p.nstages = (int)((K + BK - 1) / BK);
     p.chunk = out_dtype == TTB_FLOAT32 ? 1 : 4;
