@@ -93,7 +93,8 @@ int32_t ttb_free(void *dev_ptr);
 int32_t ttb_mem_info(int64_t *free_bytes, int64_t *total_bytes);
 int32_t ttb_host_alloc(void **host_ptr, size_t bytes); /* pinned host memory */
 int32_t ttb_host_free(void *host_ptr);
-/* Copies from and to pageable host memory may be complete when these return, as with the CUDA runtime; from 4 MiB on they are. */
+/* Copies from and to pageable host memory may be complete when these return, as with the CUDA runtime; large ones are (from 5 MiB
+ * to the device, 4 MiB to the host). */
 int32_t ttb_memcpy_h2d(void *dst_dev, const void *src_host, size_t bytes, void *stream);
 int32_t ttb_memcpy_d2h(void *dst_host, const void *src_dev, size_t bytes, void *stream);
 int32_t ttb_memcpy_d2d(void *dst_dev, const void *src_dev, size_t bytes, void *stream);

@@ -58,6 +58,15 @@ def test_copies_on_the_per_thread_stream_stay_on_the_callers_thread(fake):
     assert fake.cdll.fake_stream_users() > 1      # the legacy stream is the same on all of them
 
 
+@pytest.mark.parametrize("nbytes,to_device,to_host", [(4 * MB - 1, False, False), (4 * MB, False, True), (5 * MB - 1, False, True), (5 * MB, True, True)])
+def test_copies_are_staged_from_the_size_that_measured_faster(fake, nbytes, to_device, to_host):
+    dev, host = ctypes.create_string_buffer(nbytes), ctypes.create_string_buffer(nbytes)
+    for copy, dst, src, staged in ((fake.cdll.ttb_memcpy_h2d, dev, host, to_device), (fake.cdll.ttb_memcpy_d2h, host, dev, to_host)):
+        fake.cdll.fake_stream_users()
+        fake.check(copy(dst, src, nbytes, None))
+        assert (fake.cdll.fake_stream_users() > 1) == staged
+
+
 def test_a_stream_of_another_context_takes_the_plain_copy(fake):
     """Handle 0x300 belongs to a context that is not current (another device's, for instance): events of the current one cannot be
     recorded there."""
