@@ -2,7 +2,7 @@
 // weight dtype. One 256-thread block owns a 32x32 output tile and walks K one tile at a time,
 // expanding block-float weight tiles to fp32 in shared memory. It is the correctness anchor for the
 // tensor-core kernels (same operands, same fp32 accumulation) and serves what they do not cover
-// (batched block-float operands, fp32 results of very short sums); it is not meant to be fast.
+// (batched block-float operands, short sums of bfloat16 weights with fp32 or small results); it is not meant to be fast.
 #include "epilogue.cuh"
 
 namespace ttb {

@@ -1,6 +1,6 @@
 // Compute-bound matmul for large row counts (prefill): out[rows, N] = act(a[rows, K] x W[K, N] + bias) with W in
-// packed bfloat8_b / bfloat4_b tiles and rows a multiple of 128: fp32 results, and the bfloat16 results that matmul_rows.cu leaves
-// to it (many whole rounds of blocks; the rule is in matmul.cu).
+// packed bfloat8_b / bfloat4_b tiles and rows a multiple of 128: fp32 and reproducible results, and the bfloat16 results that
+// matmul_rows.cu leaves to it (nearly full rounds of blocks at short and long K ranges; the rule is prefill_is_faster in matmul.cu).
 //
 // One block owns a [128*R rows] x [128*H columns] output tile (R = H = 2 when the shape allows: 256 x 256, all of tensor
 // memory as two fp32 accumulators of 128 lanes x 256 columns; else 256 x 128 or 128 x 128) and walks K in blocks of 32:

@@ -1,5 +1,6 @@
 // Matmul for middling and large row counts (large decode batches, prompts; matmul.cu has the rule):
-// out_j[rows, N_j] = act(a[rows, K] x W_j[K, N_j] + bias_j) for up to four weights W_j that share the activation, in packed bfloat8_b / bfloat4_b tiles; rows, K and N multiples of 32.
+// out_j[rows, N_j] = act(a[rows, K] x W_j[K, N_j] + bias_j), bfloat16, for up to four weights W_j that share the activation, in packed
+// bfloat8_b / bfloat4_b tiles; rows, K and N multiples of 32.
 //
 // "Swap-AB", as in the decode kernels: the MMA's M dimension (128 TMEM lanes) runs over weight columns, its N dimension over up
 // to 256 activation rows, and a block owns 128 columns x one chunk of rows, so that a weight is expanded once per chunk (the
@@ -16,12 +17,13 @@
 // partial sums out of each other's shared memory, in block order: no scratch, the same bits every time. The tiles left after the
 // last whole round go to a second launch in that form.
 //
-// What bounds it: barrier round trips. With every copy, expansion and MMA left out, a ring of three groups still takes 215 clocks
-// per K block; all of it takes 300 clocks for 64 rows, 320 for 128, 415 for 192 and 520 for 256 (two groups in flight), of which the
-// MMAs are 64, 128, 192 and 256 (kernel counters: no pipe above 40 %). Groups of one or two K blocks were slower: 690 and 610
-// clocks for 256 rows. Before, as one to three launches of the decode and prefill kernels, and now, microseconds a launch from a
-// graph: 128 x 4096 x 14336 bfloat4_b 46.2 / 28.2, 352 x 4544 x 4672 48.2 / 22.8, 512 x 4096 x 4096 74.8 / 24.0, 512 x 1024 x 1024
-// 27.0 / 9.9, 256 x 8192 x 8192 71.6 / 39.8, 64 x 4096 x 1024 15.3 / 8.8, 1536 x 4096 x 14336 220 / 176.
+// What bounds it, from builds with parts left out, ns per K block of a block that owns its tile (148 tiles, 64 / 128 / 192 / 256 rows):
+// everything 163 / 172 / 193 / 258 (bfloat4_b 160 / 172 / 190 / 281); the parts alone: weight copies 145 (bfloat4_b 48), expansion 117
+// to 145, activation copies 112 to 146, MMAs 66 / 75 / 111 / 144, bare barriers 45 to 52. With two (256 rows) or three groups in flight
+// they overlap only in part; no pipe is busy for more than half the time (tensor pipe 51 % at 256 rows). Groups of one or two K
+// blocks were slower. Before, as one to three launches of the decode and prefill kernels, and now, microseconds a launch from a
+// graph: 128 x 4096 x 14336 bfloat4_b 46.2 / 26.2, 352 x 4544 x 4672 48.2 / 21.0, 512 x 4096 x 4096 74.8 / 21.9, 512 x 1024 x 1024
+// 25.8 / 8.6, 256 x 8192 x 8192 71.6 / 39.8, 64 x 4096 x 1024 14.2 / 8.0, 1536 x 4096 x 14336 210 / 159.
 // Every mbarrier wait is bounded; a wait that runs out raises a status word instead of hanging. No such wait begins while it
 // depends on the previous kernel (which may itself wait for other GPUs for seconds): the role waits for that kernel first.
 #include "decode_common.cuh"
