@@ -87,16 +87,15 @@ struct StreamPlan {
 // One persistent block per multiprocessor of the current device (read once per process; 148, a B200's count, where no device
 // can be asked - the plan and workspace queries also work without a GPU).
 int stream_blocks() {
-    static int cached = 0;
-    if (cached == 0) {
-        int dev = 0, sms = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
-            cached = sms;
-        else
-            cached = 148;
+    static std::atomic<int> cached{0};   // (whoever comes first; every thread finds the same)
+    int sms = cached.load(std::memory_order_relaxed);
+    if (sms == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
         (void)cudaGetLastError();
+        cached.store(sms, std::memory_order_relaxed);
     }
-    return cached;
+    return sms;
 }
 static constexpr int kStreamGran = 8;   // K-blocks per unit: no block gets a piece of a tile shorter than this
 
