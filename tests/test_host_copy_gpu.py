@@ -72,3 +72,38 @@ def test_several_threads(ttb):
     for t in threads:
         t.join()
     assert not failures, failures
+
+
+def test_copies_beside_another_threads_capture():
+    """The first large copies of a process, on a stream of their own, while another thread captures in global mode: both succeed, and the
+    graph replays. (A process of its own, so that the pinned buffers are not there yet.)"""
+    import os
+    import subprocess
+    import sys
+    code = """if True:
+        import sys, threading
+        sys.path.insert(0, %r)
+        import torch, cabi
+        lib, n = cabi.load(), 24 << 20
+        src, dst, dev = torch.randint(0, 256, (n,), dtype=torch.uint8), torch.zeros(n, dtype=torch.uint8), torch.empty(n, dtype=torch.uint8, device="cuda")
+        x, own, side = torch.zeros(1024, device="cuda"), torch.cuda.Stream(), torch.cuda.Stream()
+        torch.cuda.synchronize()
+        codes, graph = [], torch.cuda.CUDAGraph()
+
+        def work():
+            codes.append(lib.cdll.ttb_memcpy_h2d(dev.data_ptr(), src.data_ptr(), n, own.cuda_stream))
+            codes.append(lib.cdll.ttb_memcpy_d2h(dst.data_ptr(), dev.data_ptr(), n, own.cuda_stream))
+
+        with torch.cuda.graph(graph, stream=side, capture_error_mode="global"):
+            x.add_(1)
+            t = threading.Thread(target=work)
+            t.start()
+            t.join()
+            x.add_(1)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert codes == [0, 0], (codes, lib.cdll.ttb_last_error())
+        assert torch.equal(src, dst) and bool((x == 2).all())
+    """ % os.path.dirname(os.path.abspath(__file__))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
